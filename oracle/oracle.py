@@ -35,7 +35,7 @@ def build(quiet=True):
     """Compile the C restatement (and the reference-built driver when the tree exists)."""
     out = subprocess.DEVNULL if quiet else None
     subprocess.check_call(["make", "-s", "-C", HERE, "oracle"], stdout=out)
-    if os.path.isdir(REFERENCE_TREE):
+    if os.path.isdir(os.path.join(REFERENCE_TREE, "src", "fastpgm")):
         subprocess.check_call(["make", "-s", "-j8", "-C", HERE, "ref", "REF=" + REFERENCE_TREE], stdout=out)
 
 
