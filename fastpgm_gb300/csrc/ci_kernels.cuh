@@ -28,8 +28,9 @@ namespace fpgm {
 // compact kernel's global hash (lists 3-4 and 5 of WaveArgs::lists)
 // C_WIDET / C_WIDEQ / C_WIDEW: tests published for partition-parallel scoring, the
 // (test, partition) items queued for it, and the items taken
+// C_STRATA: tests counted through their shared variable sets (strata.cuh; list 6)
 enum { C_TIER0 = 0, C_TIER1, C_TIER2, C_WORK0, C_WORK1, C_WORK2, C_PART, C_WORKP, C_RETRY, C_WORKR, C_WIDET, C_WIDEQ,
-       C_WIDEW, C_COUNT };
+       C_WIDEW, C_STRATA, C_COUNT };
 static_assert(C_COUNT <= 16, "counters are cleared as 64 bytes");
 // stats[] slots (unsigned long long)
 // ST_TIMEOUT: a bounded device wait gave up (the tensor-core level-0 kernel)
@@ -137,8 +138,9 @@ struct WaveArgs {
     int32_t n_tests;
     // classified items
     uint16_t *item_vars;   // [T][2+d], Horner order: z1..zd, x, y
-    int32_t *lists;        // 6 lists of list_cap entries: tiers 0-2, partitioned items + their
-                           // strata estimates (float bits), items retried on the global hash
+    int32_t *lists;        // 7 lists of list_cap entries: tiers 0-2, partitioned items + their
+                           // strata estimates (float bits), items retried on the global hash,
+                           // shared-strata items (item << 1 | the side Z is drawn from)
     int64_t list_cap;
     // outputs
     uint8_t *flag;         // 1 independent, 0 dependent, 2 unsupported
@@ -148,6 +150,7 @@ struct WaveArgs {
     unsigned long long *stats;
     double alpha;
     BandTables bt;
+    int32_t strata_card;   // tests whose other endpoint has at most this many states go to list 6 (0: none)
     // compact tier: per-CTA global slots
     char *slot_mem;
     int64_t slot_bytes;
@@ -275,7 +278,7 @@ __global__ void classify_kernel(WaveArgs a) {
     const int d = a.d, ncols = d + 2;
     unsigned long long bytes_shared = 0, bytes_large = 0;  // algorithmic column bytes per tier group
     for (int item = blockIdx.x * blockDim.x + threadIdx.x; item < T; item += gridDim.x * blockDim.x) {
-        int x, y, z[kMaxCond];
+        int x, y, z[kMaxCond], side = 0;
         if (kSource == SRC_EXPLICIT) {
             const int32_t *tt = a.tests + (int64_t)item * ncols;
             x = tt[0];
@@ -295,6 +298,7 @@ __global__ void classify_kernel(WaveArgs a) {
                     rank -= a.cntx[e];
                     side_node = y;
                     skip = a.pyx[e];
+                    side = 1;
                 }
                 int c[kMaxCond];
                 unrank_lex(a.btab, a.deg[side_node] - 1, d, rank, c);
@@ -327,8 +331,12 @@ __global__ void classify_kernel(WaveArgs a) {
             atomicAdd(&a.stats[ST_UNSUPPORTED], 1ull);
             continue;
         }
-        const int slot = atomicAdd(&a.counters[C_TIER0 + tier], 1);
-        a.lists[tier * a.list_cap + slot] = item;
+        if (tier == 2 && (side ? dx : dy) <= a.strata_card) {
+            a.lists[6 * a.list_cap + atomicAdd(&a.counters[C_STRATA], 1)] = item << 1 | side;
+        } else {
+            const int slot = atomicAdd(&a.counters[C_TIER0 + tier], 1);
+            a.lists[tier * a.list_cap + slot] = item;
+        }
         const unsigned long long b = (unsigned long long)(2 + d) * (unsigned long long)a.var_S[x];
         if (tier < 2) bytes_shared += b; else bytes_large += b;
     }

@@ -30,6 +30,7 @@
 
 #include "ci_device.cuh"
 #include "ci_kernels.cuh"
+#include "strata.cuh"
 #include "fastpgm_gb300.h"
 #include "engine_internal.h"
 
@@ -206,6 +207,13 @@ struct fpgm_engine {
     unsigned long long live_prev[2] = {0ull, 0ull};
     bool live_next = false;             // the level just measured had few enough contributing samples
     double live_frac = 0.55;            // FPGM_LIVE_FRAC: write bitmaps below this contributing fraction
+    // shared strata of the tests beyond shared memory (strata.cuh; FPGM_STRATA=0, FPGM_WIDE=0 and the
+    // wave log keep them on the per-test kernels)
+    bool strata_on = true, strata_ready = false;
+    int64_t strata_f_n = 0;             // F's sample count
+    double strata_unit = 0.0;
+    bool strata_level = false;          // this level's waves use them
+    DevBuf strata_f, strata_tab, strata_lists, strata_pool, strata_refs, strata_used;
     bool tune_loaded = false, tune_online = true;
     std::string tune_source;
     // result
@@ -550,9 +558,11 @@ constexpr long long kMaxWaves = 1 << 20;  // bound on waves per level (each wave
 
 // Start of a wave: q = ranks per unresolved edge this wave (the host loop's rule: doubling from
 // 1, raised so the wave fills the GPU, capped by the item buffers), counters cleared.
-__global__ void wave_prep_kernel(WaveCtl *c, unsigned long long *stats, int32_t *counters, long long n_active,
-                                 long long ci_blocks, long long max_items) {
+__global__ void wave_prep_kernel(WaveCtl *c, unsigned long long *stats, int32_t *counters, StrataCounters *sc,
+                                 long long n_active, long long ci_blocks, long long max_items) {
     if (threadIdx.x < 16) counters[threadIdx.x] = 0;
+    if (sc)
+        for (int i = threadIdx.x; i < (int)(sizeof(StrataCounters) / 4); i += 32) reinterpret_cast<int32_t *>(sc)[i] = 0;
     if (threadIdx.x != 0) return;
     const long long unresolved = (long long)stats[ST_UNRESOLVED];
     stats[ST_UNRESOLVED] = 0;
@@ -715,6 +725,9 @@ extern "C" int fpgm_engine_create(int32_t device, fpgm_engine **out) {
     CK(cudaFuncSetAttribute(ci_part_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     CK(cudaFuncSetAttribute(ci_part_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     CK(cudaFuncSetAttribute(level0_gram_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    CK(cudaFuncSetAttribute(strata_count_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStrataInts * 4));
+    CK(cudaFuncSetAttribute(strata_count_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStrataInts * 4));
+    CK(cudaFuncSetAttribute(strata_test_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStrataInts * 4));
     CK(cudaFuncSetAttribute(ci_plain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     int occ = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ci_warp_kernel<kWarpInts, 2>, kThreads, kSmemBytes));
@@ -745,6 +758,7 @@ extern "C" int fpgm_engine_create(int32_t device, fpgm_engine **out) {
     if (const char *w = getenv("FPGM_WIDE")) e->wide_on = atoi(w) != 0;
     if (const char *w = getenv("FPGM_GRAM")) e->gram_on = atoi(w) != 0;
     if (const char *w = getenv("FPGM_GRAPH")) e->graph_on = atoi(w) != 0;
+    if (const char *w = getenv("FPGM_STRATA")) e->strata_on = atoi(w) != 0;
     e->gram = gram_create();
     if (const char *w = getenv("FPGM_WIDE_N2")) e->wide_small_n2 = atoi(w);
     if (const char *w = getenv("FPGM_WIDE_MIN_LOG")) e->wide_min_log = std::min(kPartMaxLog, std::max(0, atoi(w)));
@@ -789,7 +803,8 @@ extern "C" int fpgm_engine_destroy(fpgm_engine *e) {
                       &e->mle_pot, &e->mle_meta, &e->wide, &e->wide_items, &e->tune, &e->wave_ctl,
                       &e->tune_obs, &e->ovf, &e->live_pool[0], &e->live_pool[1], &e->live_tab[0], &e->live_tab[1],
                       &e->live_cnt, &e->live_stat, &e->res_adj_d, &e->res_key, &e->res_idx, &e->res_removed_d, &e->res_cnt,
-                      &e->res_vars_d};
+                      &e->res_vars_d, &e->strata_f, &e->strata_tab, &e->strata_lists, &e->strata_pool,
+                      &e->strata_refs, &e->strata_used};
     for (DevBuf *b : bufs) b->release();
     gram_destroy(e->gram);
     if (e->ev0) cudaEventDestroy(e->ev0);
@@ -1003,6 +1018,116 @@ int live_setup(fpgm_engine *e, int d) {
     return FPGM_OK;
 }
 
+// ---- shared strata (strata.cuh)
+// Tables: keys of nodes and pairs, then their fields; all sized by the two capacities.
+constexpr int kStrataNodes = 1 << 19, kStrataPairs = 1 << 20, kStrataBuild = 1 << 17;
+constexpr size_t kStrataKeyBytes = (size_t)kStrataNodes * 8 + (size_t)kStrataPairs * 8;
+
+void strata_args(fpgm_engine *e, StrataArgs &s) {
+    memset(&s, 0, sizeof s);
+    char *t = e->strata_tab.as<char>();
+    auto take = [&](size_t bytes) {
+        char *p = t;
+        t += bytes;
+        return p;
+    };
+    s.node_key = reinterpret_cast<uint64_t *>(take((size_t)kStrataNodes * 8));
+    s.pair_key = reinterpret_cast<uint64_t *>(take((size_t)kStrataPairs * 8));
+    s.node_h = reinterpret_cast<long long *>(take((size_t)kStrataNodes * 8));
+    s.node_ids = reinterpret_cast<int64_t *>(take((size_t)kStrataNodes * 8));
+    s.pair_h = reinterpret_cast<long long *>(take((size_t)kStrataPairs * 8));
+    s.pair_a = reinterpret_cast<int64_t *>(take((size_t)kStrataPairs * 8));
+    s.node_n = reinterpret_cast<int32_t *>(take((size_t)kStrataNodes * 4));
+    s.node_max = reinterpret_cast<int32_t *>(take((size_t)kStrataNodes * 4));
+    s.node_cap = kStrataNodes;
+    s.pair_cap = kStrataPairs;
+    s.pool = e->strata_pool.as<char>();
+    s.pool_cap = e->strata_pool.bytes;
+    s.pool_used = e->strata_used.as<unsigned long long>();
+    s.sc = reinterpret_cast<StrataCounters *>(e->strata_used.as<char>() + 64);
+    s.build_list = e->strata_lists.as<int32_t>();
+    s.build_cap = kStrataBuild;
+    s.pair_list = s.build_list + (size_t)(kStrataMaxSets + 1) * kStrataBuild;
+    s.pair_list_cap = kStrataPairs;
+    s.item_ref = e->strata_refs.as<int4>();
+    s.f = e->strata_f.as<long long>();
+    s.unit = e->strata_unit;
+    // 2 S counts of two or more at most over the four sums, half a unit each, doubled; and the
+    // FP64 rounding of the largest F
+    s.err = 2.0 * e->strata_unit + 1e-14;
+}
+
+// Level d's waves count through shared strata when a test can go past shared memory: buffers
+// made (or, when the last level came near their end, grown and emptied).  No room: not used.
+int strata_setup(fpgm_engine *e, int d, bool first) {
+    e->strata_level = false;
+    if (first) e->strata_ready = false;
+    if (!e->strata_on || !e->wide_on || e->wave_log || e->phase_timers.p || e->S > kStrataMaxSamples || d < 1 ||
+        d + 1 > kStrataMaxSets || max_table_ints(e->h_card, d) <= kCtaInts - 64)
+        return FPGM_OK;
+    const size_t tab = kStrataKeyBytes + (size_t)kStrataNodes * 24 + (size_t)kStrataPairs * 16;
+    const size_t slot = (size_t)((e->S + 15) & ~(int64_t)15) * 2;
+    unsigned long long used[3] = {0, 0, 0};
+    if (e->strata_ready) {
+        CK(cudaMemcpyAsync(used, e->strata_used.p, sizeof used, cudaMemcpyDeviceToHost, e->stream));
+        CK(cudaStreamSynchronize(e->stream));
+    }
+    bool empty = !e->strata_ready;
+    const size_t least = std::max<size_t>((size_t)256 << 20, slot * 8192);
+    size_t want = std::max(least, e->strata_pool.bytes);
+    if (e->strata_ready && used[0] > e->strata_pool.bytes / 2) want = std::max(want, 4 * e->strata_pool.bytes);
+    if (want > e->strata_pool.bytes) {
+        size_t free_b = 0, total_b = 0;
+        CK(cudaMemGetInfo(&free_b, &total_b));
+        want = std::min(want, std::max(least, (size_t)std::min(32.0e9, 0.25 * (double)(free_b + e->strata_pool.bytes))));
+        if (want > e->strata_pool.bytes + e->strata_pool.bytes / 4) {
+            e->strata_pool.release();
+            empty = true;
+            if (e->strata_pool.ensure(want) != FPGM_OK && e->strata_pool.ensure(least) != FPGM_OK) {
+                e->strata_on = false;  // no room: the per-test kernels
+                return FPGM_OK;
+            }
+        }
+    }
+    if (used[0] > e->strata_pool.bytes / 2 || used[1] > kStrataNodes / 3 || used[2] > kStrataPairs / 3) empty = true;
+    if (e->strata_tab.ensure(tab) != FPGM_OK ||
+        e->strata_lists.ensure(((size_t)(kStrataMaxSets + 1) * kStrataBuild + kStrataPairs) * 4) != FPGM_OK ||
+        e->strata_used.ensure(64 + sizeof(StrataCounters)) != FPGM_OK) {
+        e->strata_on = false;
+        return FPGM_OK;
+    }
+    if (e->strata_f_n < e->S) {
+        RET(e->strata_f.ensure((size_t)(e->S + 1) * 8));
+        const double top = (double)e->S * log((double)std::max<int64_t>(e->S, 3));
+        const int k = 59 - (int)ceil(log2(top));  // four sums of at most `top` stay below 2^61
+        e->strata_unit = ldexp(1.0, -k);
+        strata_f_kernel<<<blocks_for(e->S + 1, 256), 256, 0, e->stream>>>(e->strata_f.as<long long>(), e->S,
+                                                                         ldexp(1.0, k));
+        CK(cudaGetLastError());
+        e->strata_f_n = e->S;
+        empty = true;  // sums of another unit
+    }
+    if (empty) {
+        CK(cudaMemsetAsync(e->strata_tab.p, 0, kStrataKeyBytes, e->stream));
+        CK(cudaMemsetAsync(e->strata_used.p, 0, 64, e->stream));
+    }
+    e->strata_ready = e->strata_level = true;
+    return FPGM_OK;
+}
+
+// The shared-strata kernels of one wave on the current stream.  Returns launches issued.
+int launch_strata(fpgm_engine *e, const WaveArgs &a) {
+    StrataArgs s;
+    strata_args(e, s);
+    strata_collect_kernel<<<e->ci_blocks, 128, 0, e->stream>>>(a, s);
+    const int grid = 2 * e->num_sms;
+    for (int size = 1; size <= a.d + 1; ++size)
+        strata_count_kernel<true><<<grid, kStrataThreads, kStrataInts * 4, e->stream>>>(a, s, size);
+    strata_count_kernel<false><<<grid, kStrataThreads, kStrataInts * 4, e->stream>>>(a, s, 0);
+    strata_test_kernel<<<grid, kStrataThreads, kStrataInts * 4, e->stream>>>(a, s);
+    return a.d + 4;
+}
+
 int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t items) {
     memset(&a, 0, sizeof a);
     a.cols = e->cols.as<uint8_t>();
@@ -1019,7 +1144,7 @@ int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t ite
     a.bt.hi = a.bt.lo + kBandDfMax + 1;
     a.bt.dfmax = kBandDfMax;
     RET(e->item_vars.ensure((size_t)std::max<int64_t>(items, 1) * (2 + d) * 2 + 16));
-    RET(e->lists.ensure((size_t)6 * std::max<int64_t>(items, 1) * 4 + 16));
+    RET(e->lists.ensure((size_t)7 * std::max<int64_t>(items, 1) * 4 + 16));
     RET(e->flag.ensure((size_t)std::max<int64_t>(items, 1) + 16));
     a.item_vars = e->item_vars.as<uint16_t>();
     a.lists = e->lists.as<int32_t>();
@@ -1060,6 +1185,10 @@ int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t ite
                 a.bm_prev_tab_cap = e->live_tab_cap;
             }
         }
+    }
+    if (e->strata_level && d >= 1) {
+        RET(e->strata_refs.ensure((size_t)std::max<int64_t>(items, 1) * sizeof(int4)));
+        a.strata_card = kStrataMaxCard;
     }
     a.part_max_log = e->part_max_log;
     a.warp_ints = e->warp_small ? kWarpIntsSmall : kWarpInts;
@@ -1151,7 +1280,10 @@ int run_waves_graph(fpgm_engine *e, double alpha, int d, int64_t n_active, fpgm_
         CK(cudaGraphAddNode(&cn, graph, nullptr, nullptr, 0, &cp));
         cudaGraph_t body = cp.conditional.phGraph_out[0];
         CK(cudaStreamBeginCaptureToGraph(e->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-        wave_prep_kernel<<<1, 32, 0, e->stream>>>(ctl, dstat, e->counters.as<int32_t>(), (long long)n_active,
+        StrataArgs sa;
+        strata_args(e, sa);
+        wave_prep_kernel<<<1, 32, 0, e->stream>>>(ctl, dstat, e->counters.as<int32_t>(),
+                                                  a.strata_card ? sa.sc : nullptr, (long long)n_active,
                                                   (long long)e->ci_blocks, (long long)kMaxItems);
         wave_plan_dev_kernel<<<blocks_for(n_active + 1, 256), 256, 0, e->stream>>>(
             (int)n_active, e->status.as<uint8_t>(), e->total.as<uint64_t>(), e->next.as<uint64_t>(), ctl,
@@ -1164,6 +1296,7 @@ int run_waves_graph(fpgm_engine *e, double alpha, int d, int64_t n_active, fpgm_
         ci_cta_kernel<<<e->ci_blocks, kThreads, kSmemBytes, e->stream>>>(a);
         wave_stamp_kernel<<<1, 1, 0, e->stream>>>(ctl, 0);
         per_wave = 9;  // prep, plan, 3 stamps, classify, warp tier, CTA tier, reduce, tail (+ tier 2)
+        if (a.strata_card) per_wave += launch_strata(e, a);
         if (a.slot_mem) per_wave += launch_compact(e, a, e->n_slots);
         wave_stamp_kernel<<<1, 1, 0, e->stream>>>(ctl, 1);
         wave_reduce_kernel<<<blocks_for(n_active, 256), 256, 0, e->stream>>>(
@@ -1268,6 +1401,12 @@ int run_waves_and_count(fpgm_engine *e, double alpha, int d, int64_t n_active, f
         }
         CK(cudaEventRecord(e->ev1, e->stream));
         a.dbg = e->phase_timers.as<unsigned long long>();
+        if (a.strata_card && !gram) {
+            StrataArgs sa;
+            strata_args(e, sa);
+            CK(cudaMemsetAsync(sa.sc, 0, sizeof(StrataCounters), e->stream));
+            st->kernel_launches += launch_strata(e, a);
+        }
         if (a.slot_mem && !gram) {
             st->kernel_launches += launch_compact(e, a, e->n_slots);
             CK(cudaGetLastError());
@@ -1364,6 +1503,7 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
         }
         ~LiveScope() {
             e->live_level[0] = e->live_level[1] = -1;
+            e->strata_level = false;
             e->live_write = false;
             e->live_in_skeleton = false;
         }
@@ -1482,6 +1622,7 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
                 gram = e->gram_ok;
             }
             if (!gram) RET(live_setup(e, d));
+            RET(strata_setup(e, d, d <= 1));
             RET(run_waves_and_count(e, alpha, d, n_active, st, st->n_levels, a, gram));
             if (e->live_on && e->live_stat.p) {
                 // Bitmaps pay for themselves when the next level can leave enough samples out:
