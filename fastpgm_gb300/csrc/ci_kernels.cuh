@@ -20,6 +20,7 @@
 // then summed into the dense table.
 #pragma once
 #include "ci_device.cuh"
+#include "fixed.cuh"
 
 namespace fpgm {
 
@@ -28,10 +29,13 @@ namespace fpgm {
 // compact kernel's global hash (lists 3-4 and 5 of WaveArgs::lists)
 // C_WIDET / C_WIDEQ / C_WIDEW: tests published for partition-parallel scoring, the
 // (test, partition) items queued for it, and the items taken
+// C_SETW / C_SETC: variable sets to count by a warp / a CTA, C_SCOREW / C_SCOREC: tests to score
+// from their set's table by a warp / a CTA, and the ones taken (sets.cuh)
 // C_STRATA: tests counted through their shared variable sets (strata.cuh; list 6)
 enum { C_TIER0 = 0, C_TIER1, C_TIER2, C_WORK0, C_WORK1, C_WORK2, C_PART, C_WORKP, C_RETRY, C_WORKR, C_WIDET, C_WIDEQ,
-       C_WIDEW, C_STRATA, C_COUNT };
-static_assert(C_COUNT <= 16, "counters are cleared as 64 bytes");
+       C_WIDEW, C_STRATA, C_SETW, C_WSETW, C_SETC, C_WSETC, C_SCOREW, C_WSCOREW, C_SCOREC, C_WSCOREC, C_COUNT };
+constexpr int kCounterBytes = 128;
+static_assert(C_COUNT * 4 <= kCounterBytes, "counters are cleared together");
 // stats[] slots (unsigned long long)
 // ST_TIMEOUT: a bounded device wait gave up (the tensor-core level-0 kernel)
 enum { ST_RECHECK = 0, ST_NEARTIE, ST_LARGE, ST_MAXDP, ST_UNSUPPORTED, ST_DET, ST_EXEC, ST_UNRESOLVED,
@@ -118,6 +122,21 @@ __device__ inline int live_find(const LiveKey *tab, int cap, const uint16_t *v, 
     return -1;
 }
 
+// Tables counted once per variable set (sets.cuh), kept for a level.
+struct SetArgs {
+    uint64_t *key;             // open addressing; null: every test counts its own table
+    int32_t cap;               // power of two
+    int32_t probe;             // places tried before a set goes without
+    int32_t *off;              // per entry: its table's first int in the pool
+    long long *h;              // per entry: sum of F over its cells
+    int32_t *pool;
+    unsigned long long pool_cap;
+    unsigned long long *used;  // ints of the pool handed out
+    int2 *fresh;               // sets to count (entry, an item): a warp's from the front, a CTA's from the end
+    int2 *items;               // tests to score (entry, item), likewise
+    int32_t few;               // at most this many new sets: each is counted by a CTA
+};
+
 struct WaveArgs {
     const uint8_t *cols;
     const int64_t *var_off;  // byte offset of each variable's column in cols
@@ -150,6 +169,8 @@ struct WaveArgs {
     unsigned long long *stats;
     double alpha;
     BandTables bt;
+    Fixed fx;              // fixed-point statistic of tests that need no detail
+    SetArgs sets;
     int32_t strata_card;   // tests whose other endpoint has at most this many states go to list 6 (0: none)
     // compact tier: per-CTA global slots
     char *slot_mem;
@@ -271,6 +292,41 @@ __device__ inline int upper_bound_i32(const int32_t *a, int n, int v) {
     return lo;
 }
 
+__device__ __forceinline__ uint64_t key_cas(uint64_t *p, uint64_t e, uint64_t v) {
+    return atomicCAS(reinterpret_cast<unsigned long long *>(p), (unsigned long long)e, (unsigned long long)v);
+}
+__device__ __forceinline__ uint32_t key_cas(uint32_t *p, uint32_t e, uint32_t v) { return atomicCAS(p, e, v); }
+
+// Place of a nonzero key in an open-addressing table (entered when absent: *fresh); -1 after
+// that many places.
+constexpr int kEnterProbe = 128;
+__device__ inline int table_enter(uint64_t *keys, int cap, int probe, uint64_t key, bool *fresh) {
+    uint32_t h = (uint32_t)((key * 0x9E3779B97F4A7C15ull) >> 32) & (uint32_t)(cap - 1);
+    *fresh = false;
+    for (int p = 0; p < probe; ++p) {
+        uint64_t k = *(volatile uint64_t *)&keys[h];
+        if (k == key) return (int)h;
+        if (k == 0) {
+            k = key_cas(&keys[h], 0ull, key);
+            if (k == 0) *fresh = true;
+            if (k == 0 || k == key) return (int)h;
+        }
+        h = (h + 1) & (uint32_t)(cap - 1);
+    }
+    return -1;
+}
+
+// Entry of the set of m >= 3 ascending variables: the first three in one key, then two at a
+// time after the entry reached so far (the keys hold the variables themselves, so two sets
+// never share an entry).  -1: no room.
+__device__ inline int set_enter(const SetArgs &s, const uint16_t *v, int m, bool *fresh) {
+    int at = table_enter(s.key, s.cap, s.probe, (1ull << 62) | (uint64_t)v[0] << 32 | (uint64_t)v[1] << 16 | v[2], fresh);
+    for (int i = 3; i < m && at >= 0; i += 2)
+        at = table_enter(s.key, s.cap, s.probe,
+                         (1ull << 63) | (uint64_t)at << 32 | (uint64_t)v[i] << 16 | (i + 1 < m ? v[i + 1] : 0xffffu), fresh);
+    return at;
+}
+
 // Item -> (x, y, Z) -> tier.  One thread per item, grid-stride.
 template <int kSource>
 __global__ void classify_kernel(WaveArgs a) {
@@ -331,7 +387,40 @@ __global__ void classify_kernel(WaveArgs a) {
             atomicAdd(&a.stats[ST_UNSUPPORTED], 1ull);
             continue;
         }
-        if (tier == 2 && (side ? dx : dy) <= a.strata_card) {
+        bool placed = false;
+        if (kSource == SRC_WAVE && tier < 2 && a.sets.key != nullptr && d > 0) {
+            uint16_t sv[kMaxCols];  // the set, ascending (x < y, z ascending)
+            for (int k = 0, i = 0, j = 0; k < ncols; ++k) {
+                const int p = j == 0 ? x : y;
+                if (j < 2 && (i == d || p < z[i])) {
+                    sv[k] = (uint16_t)p;
+                    ++j;
+                } else {
+                    sv[k] = (uint16_t)z[i++];
+                }
+            }
+            const int cells = (int)dz * dx * dy, work = cells + (int)dz * (dx + dy + 2);
+            bool fresh;
+            const int at = work > kCtaInts ? -1 : set_enter(a.sets, sv, ncols, &fresh);
+            if (at >= 0) {
+                if (fresh) {
+                    const unsigned long long o = atomicAdd(a.sets.used, (unsigned long long)((cells + 3) & ~3));
+                    const bool room = o + cells <= a.sets.pool_cap;
+                    a.sets.off[at] = room ? (int32_t)o : -1;
+                    if (room) {
+                        const bool warp = cells <= a.warp_ints;
+                        const int q = atomicAdd(&a.counters[warp ? C_SETW : C_SETC], 1);
+                        a.sets.fresh[warp ? q : a.list_cap - 1 - q] = make_int2(at, item);
+                    }
+                }
+                const bool warp = work <= a.warp_ints;
+                const int q = atomicAdd(&a.counters[warp ? C_SCOREW : C_SCOREC], 1);
+                a.sets.items[warp ? q : a.list_cap - 1 - q] = make_int2(at, item);
+                placed = true;
+            }
+        }
+        if (placed) {
+        } else if (tier == 2 && (side ? dx : dy) <= a.strata_card) {
             a.lists[6 * a.list_cap + atomicAdd(&a.counters[C_STRATA], 1)] = item << 1 | side;
         } else {
             const int slot = atomicAdd(&a.counters[C_TIER0 + tier], 1);
@@ -373,6 +462,41 @@ __device__ __forceinline__ void horner_pair(uint32_t (&ca)[8], uint32_t (&cb)[8]
             horner16(ca, wa[t], dim[j0 + t]);
             horner16(cb, wb[t], dim[j0 + t]);
         }
+    }
+}
+
+// Adds the samples of ncols columns (Horner order) to a table of 2^lgR replicas interleaved cell
+// by cell (cell c of replica r at c << lgR | r; this lane's is lane mod 2^lgR).  Called by
+// kStep threads, t = 0 .. kStep - 1.  Two samples share a 32-bit register until the end, where
+// one dot-product instruction takes a 16-bit code to its shared-memory address.
+template <int kStep>
+__device__ __forceinline__ void count_columns(int *rep, int lgR, int lane, const uint8_t *const *col,
+                                              const uint32_t *dim, int ncols, int64_t S, int t) {
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(rep + (lane & ((1 << lgR) - 1)));
+    const uint32_t mlo = 4u << lgR, mhi = mlo << 8;
+    const int64_t nvec = S >> 4;
+    auto add = [](uint32_t at) { asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(at) : "memory"); };
+    for (int64_t v = t; v < nvec; v += 2 * kStep) {
+        const bool two = v + kStep < nvec;
+        uint32_t ca[8], cb[8];
+        horner_pair(ca, cb, col, dim, ncols, v, v + kStep, two);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            add(__dp2a_lo(ca[q], mlo, base));
+            add(__dp2a_lo(ca[q], mhi, base));
+        }
+        if (two) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                add(__dp2a_lo(cb[q], mlo, base));
+                add(__dp2a_lo(cb[q], mhi, base));
+            }
+        }
+    }
+    for (int64_t s = (S & ~(int64_t)15) + t; s < S; s += kStep) {
+        uint32_t c = 0;
+        for (int j = 0; j < ncols; ++j) c = c * dim[j] + col[j][s];
+        add(base + (c << lgR << 2));
     }
 }
 
@@ -419,7 +543,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) ci_warp_kernel(WaveArgs 
         if (idx >= n0) break;
         const int item = a.lists[idx];
         const int64_t S = a.var_S[a.item_vars[(int64_t)item * ncols + d]];
-        const int64_t nvec = S >> 4;
         uint32_t dim = 1;
         if (lane < ncols) {
             const int var = a.item_vars[(int64_t)item * ncols + lane];
@@ -443,31 +566,9 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) ci_warp_kernel(WaveArgs 
         int *ni = tab + cells, *nj = ni + dz * dx, *nk = nj + dz * dy;
         for (int i = lane; i < ((int)cells << lgR); i += 32) rep[i] = 0;
         __syncwarp();
-        // lane l counts into replica l mod R: with 32 replicas every lane owns one bank, so a
-        // warp's 32 increments never conflict whatever cells they hit
-        int *myrep = rep + (lane & (R - 1));
-        for (int64_t v = lane; v < nvec; v += 64) {
-            const bool two = v + 32 < nvec;
-            uint32_t ca[8], cb[8];
-            horner_pair(ca, cb, s_col[warp], s_dim[warp], ncols, v, v + 32, two);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                atomicAdd(&myrep[(ca[q] & 0xffffu) << lgR], 1);
-                atomicAdd(&myrep[(ca[q] >> 16) << lgR], 1);
-            }
-            if (two) {
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    atomicAdd(&myrep[(cb[q] & 0xffffu) << lgR], 1);
-                    atomicAdd(&myrep[(cb[q] >> 16) << lgR], 1);
-                }
-            }
-        }
-        for (int64_t s = (S & ~(int64_t)15) + lane; s < S; s += 32) {
-            uint32_t c = 0;
-            for (int j = 0; j < ncols; ++j) c = c * s_dim[warp][j] + s_col[warp][j][s];
-            atomicAdd(&myrep[c << lgR], 1);
-        }
+        // with 32 replicas every lane owns one bank, so a warp's 32 increments never conflict
+        // whatever cells they hit
+        count_columns<32>(rep, lgR, lane, s_col[warp], s_dim[warp], ncols, S, lane);
         __syncwarp();
         if (R > 1) {
             for (int c = lane; c < (int)cells; c += 32) {
@@ -502,7 +603,6 @@ __global__ void __launch_bounds__(kThreads, 2) ci_cta_kernel(WaveArgs a) {
         if (idx >= n1) break;
         const int item = a.lists[a.list_cap + idx];
         const int64_t S = a.var_S[a.item_vars[(int64_t)item * ncols + d]];
-        const int64_t nvec = S >> 4;
         if (tid < ncols) {
             const int var = a.item_vars[(int64_t)item * ncols + tid];
             s_dim[tid] = a.card[var];
@@ -523,29 +623,7 @@ __global__ void __launch_bounds__(kThreads, 2) ci_cta_kernel(WaveArgs a) {
         int *ni = tab + cells, *nj = ni + dz * dx, *nk = nj + dz * dy;
         for (int i = tid; i < (cells << lgR); i += kThreads) rep[i] = 0;
         __syncthreads();
-        int *myrep = rep + (lane & (R - 1));
-        for (int64_t v = tid; v < nvec; v += 2 * kThreads) {
-            const bool two = v + kThreads < nvec;
-            uint32_t ca[8], cb[8];
-            horner_pair(ca, cb, s_col, s_dim, ncols, v, v + kThreads, two);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                atomicAdd(&myrep[(ca[q] & 0xffffu) << lgR], 1);
-                atomicAdd(&myrep[(ca[q] >> 16) << lgR], 1);
-            }
-            if (two) {
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    atomicAdd(&myrep[(cb[q] & 0xffffu) << lgR], 1);
-                    atomicAdd(&myrep[(cb[q] >> 16) << lgR], 1);
-                }
-            }
-        }
-        for (int64_t s = (S & ~(int64_t)15) + tid; s < S; s += kThreads) {
-            uint32_t c = 0;
-            for (int j = 0; j < ncols; ++j) c = c * s_dim[j] + s_col[j][s];
-            atomicAdd(&myrep[c << lgR], 1);
-        }
+        count_columns<kThreads>(rep, lgR, lane, s_col, s_dim, ncols, S, tid);
         __syncthreads();
         if (R > 1) {
             for (int c = tid; c < cells; c += kThreads) {
@@ -593,11 +671,6 @@ __device__ __forceinline__ uint32_t zhash(uint64_t z, uint32_t cap) {
 // Inserts stratum code z; a new code takes the next id from *counter, written to ids[slot]
 // (16- or 32-bit ids) and, when gzk is given, its code to gzk[id].  Returns the slot, or -1
 // after max_probe probes or once more than id_limit strata exist.
-__device__ __forceinline__ uint64_t key_cas(uint64_t *p, uint64_t e, uint64_t v) {
-    return atomicCAS(reinterpret_cast<unsigned long long *>(p), (unsigned long long)e, (unsigned long long)v);
-}
-__device__ __forceinline__ uint32_t key_cas(uint32_t *p, uint32_t e, uint32_t v) { return atomicCAS(p, e, v); }
-
 template <class K, class Id>
 __device__ inline int zinsert(K *keys, Id *ids, uint32_t cap, uint64_t zz, int *counter, int id_limit,
                               uint32_t max_probe, uint64_t *gzk) {
@@ -2750,16 +2823,11 @@ __global__ void __launch_bounds__(kThreads, 2) ci_part_wide_kernel(WaveArgs a) {
 }
 
 // ---------------------------------------------------------------- band tables
-__global__ void band_table_kernel(double alpha, double *lo, double *hi, int dfmax) {
-    const int df = blockIdx.x * blockDim.x + threadIdx.x;
+// Two threads per df: one quantile each (latency, not throughput, bounds the table).
+__global__ void band_table_kernel(double alpha, double band, double *lo, double *hi, int dfmax) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, df = i >> 1;
     if (df > dfmax) return;
-    if (df == 0) {
-        lo[0] = 0.0;
-        hi[0] = 0.0;
-        return;
-    }
-    lo[df] = chisq_quantile_upper(alpha + kBand, df);
-    hi[df] = chisq_quantile_upper(alpha - kBand, df);
+    (i & 1 ? hi : lo)[df] = df == 0 ? 0.0 : chisq_quantile_upper(i & 1 ? alpha - band : alpha + band, df);
 }
 
 // ---------------------------------------------------------------- plain: one test, whole grid, one launch

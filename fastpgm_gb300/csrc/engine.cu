@@ -30,6 +30,7 @@
 
 #include "ci_device.cuh"
 #include "ci_kernels.cuh"
+#include "sets.cuh"
 #include "strata.cuh"
 #include "fastpgm_gb300.h"
 #include "engine_internal.h"
@@ -210,10 +211,22 @@ struct fpgm_engine {
     // shared strata of the tests beyond shared memory (strata.cuh; FPGM_STRATA=0, FPGM_WIDE=0 and the
     // wave log keep them on the per-test kernels)
     bool strata_on = true, strata_ready = false;
-    int64_t strata_f_n = 0;             // F's sample count
-    double strata_unit = 0.0;
     bool strata_level = false;          // this level's waves use them
-    DevBuf strata_f, strata_tab, strata_lists, strata_pool, strata_refs, strata_used;
+    DevBuf strata_tab, strata_lists, strata_pool, strata_refs, strata_used;
+    // fixed-point statistic (fixed.cuh) and tables per variable set (sets.cuh; FPGM_SETS=0: none)
+    DevBuf fixed_f, tight;
+    int64_t fixed_n = 0;                // F's sample count
+    double fixed_unit = 0.0;
+    double tight_alpha = -1.0;
+    int tight_df = 0, band_df = 0;      // degrees of freedom the quantile tables reach
+    bool in_skeleton = false;           // a batched skeleton's waves (decisions only)
+    bool sets_on = true, sets_level = false;
+    bool sets_all = false;              // ... and there is room for every set of the level
+    int32_t sets_cap = 0;
+    int64_t level_tests = 0;            // bound of the level's tests
+    unsigned long long sets_used = 0;   // ints of tables the last level asked for
+    size_t set_pool_fixed = 0, strata_pool_fixed = 0;  // FPGM_SET_POOL, FPGM_STRATA_POOL (tests): bytes
+    DevBuf set_tab, set_pool, set_items;
     bool tune_loaded = false, tune_online = true;
     std::string tune_source;
     // result
@@ -560,7 +573,7 @@ constexpr long long kMaxWaves = 1 << 20;  // bound on waves per level (each wave
 // 1, raised so the wave fills the GPU, capped by the item buffers), counters cleared.
 __global__ void wave_prep_kernel(WaveCtl *c, unsigned long long *stats, int32_t *counters, StrataCounters *sc,
                                  long long n_active, long long ci_blocks, long long max_items) {
-    if (threadIdx.x < 16) counters[threadIdx.x] = 0;
+    counters[threadIdx.x] = 0;  // 32 threads, kCounterBytes
     if (sc)
         for (int i = threadIdx.x; i < (int)(sizeof(StrataCounters) / 4); i += 32) reinterpret_cast<int32_t *>(sc)[i] = 0;
     if (threadIdx.x != 0) return;
@@ -648,9 +661,10 @@ __global__ void __launch_bounds__(kThreads) level0_gram_score_kernel(WaveArgs a,
                 if (c0 + 32 * u + lane < cells) tab[c0 + 32 * u + lane] = v[u];
         }
         __syncwarp();
-        const Verdict v = score_dense(g, tab, ni, nj, nk, dx, dy, 1, a.alpha, a.bt, a.detail != nullptr,
-                                      a.want_hash != 0, nullptr);
-        if (lane == 0) record(a, item, v, cells, a.want_hash ? table_hash(tab, cells) : 0, 0);
+        const Verdict v = a.fx.f ? score_fixed(g, tab, nullptr, dy, 1, dx, dy, 1, ni, nj, nk, nullptr, a.fx, a.alpha,
+                                               a.var_S[x], nullptr)
+                                 : score_dense(g, tab, ni, nj, nk, dx, dy, 1, a.alpha, a.bt, false, false, nullptr);
+        if (lane == 0) record(a, item, v, cells, 0, 0);
         __syncwarp();
     }
 }
@@ -727,6 +741,14 @@ extern "C" int fpgm_engine_create(int32_t device, fpgm_engine **out) {
     CK(cudaFuncSetAttribute(level0_gram_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     CK(cudaFuncSetAttribute(strata_count_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStrataInts * 4));
     CK(cudaFuncSetAttribute(strata_count_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStrataInts * 4));
+    CK(cudaFuncSetAttribute(set_count_warp_kernel<kWarpInts, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    CK(cudaFuncSetAttribute(set_score_warp_kernel<kWarpInts, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    CK(cudaFuncSetAttribute(set_count_warp_kernel<kWarpIntsSmall, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            kWarps * kWarpIntsSmall * 4));
+    CK(cudaFuncSetAttribute(set_score_warp_kernel<kWarpIntsSmall, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            kWarps * kWarpIntsSmall * 4));
+    CK(cudaFuncSetAttribute(set_count_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    CK(cudaFuncSetAttribute(set_score_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     CK(cudaFuncSetAttribute(strata_test_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStrataInts * 4));
     CK(cudaFuncSetAttribute(ci_plain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     int occ = 0;
@@ -751,7 +773,7 @@ extern "C" int fpgm_engine_create(int32_t device, fpgm_engine **out) {
     }
     RET(e->btab.ensure(bt.size() * 8));
     CK(cudaMemcpy(e->btab.p, bt.data(), bt.size() * 8, cudaMemcpyHostToDevice));
-    RET(e->counters.ensure(64));
+    RET(e->counters.ensure(kCounterBytes));
     RET(e->stats.ensure(ST_COUNT * 8));
     e->wave_log = getenv("FPGM_WAVE_LOG") != nullptr;
     if (const char *pm = getenv("FPGM_PART_MAX_LOG")) e->part_max_log = std::min(kPartMaxLog, std::max(1, atoi(pm)));
@@ -759,6 +781,9 @@ extern "C" int fpgm_engine_create(int32_t device, fpgm_engine **out) {
     if (const char *w = getenv("FPGM_GRAM")) e->gram_on = atoi(w) != 0;
     if (const char *w = getenv("FPGM_GRAPH")) e->graph_on = atoi(w) != 0;
     if (const char *w = getenv("FPGM_STRATA")) e->strata_on = atoi(w) != 0;
+    if (const char *w = getenv("FPGM_SETS")) e->sets_on = atoi(w) != 0;
+    if (const char *w = getenv("FPGM_SET_POOL")) e->set_pool_fixed = (size_t)std::max(16ll, atoll(w));
+    if (const char *w = getenv("FPGM_STRATA_POOL")) e->strata_pool_fixed = (size_t)std::max(16ll, atoll(w));
     e->gram = gram_create();
     if (const char *w = getenv("FPGM_WIDE_N2")) e->wide_small_n2 = atoi(w);
     if (const char *w = getenv("FPGM_WIDE_MIN_LOG")) e->wide_min_log = std::min(kPartMaxLog, std::max(0, atoi(w)));
@@ -803,7 +828,8 @@ extern "C" int fpgm_engine_destroy(fpgm_engine *e) {
                       &e->mle_pot, &e->mle_meta, &e->wide, &e->wide_items, &e->tune, &e->wave_ctl,
                       &e->tune_obs, &e->ovf, &e->live_pool[0], &e->live_pool[1], &e->live_tab[0], &e->live_tab[1],
                       &e->live_cnt, &e->live_stat, &e->res_adj_d, &e->res_key, &e->res_idx, &e->res_removed_d, &e->res_cnt,
-                      &e->res_vars_d, &e->strata_f, &e->strata_tab, &e->strata_lists, &e->strata_pool,
+                      &e->res_vars_d, &e->fixed_f, &e->tight, &e->set_tab,
+                      &e->set_pool, &e->set_items, &e->strata_tab, &e->strata_lists, &e->strata_pool,
                       &e->strata_refs, &e->strata_used};
     for (DevBuf *b : bufs) b->release();
     gram_destroy(e->gram);
@@ -922,16 +948,26 @@ extern "C" int fpgm_dataset_download(fpgm_engine *e, uint8_t *columns) {
 // ------------------------------------------------------------------ batched skeleton
 namespace {
 
-// Band-edge tables for alpha (cached per alpha).
-int ensure_band(fpgm_engine *e, double alpha) {
-    if (e->band_alpha == alpha && e->band.p) return FPGM_OK;
-    RET(e->band.ensure((size_t)2 * (kBandDfMax + 1) * sizeof(double)));
-    double *lo = e->band.as<double>(), *hi = lo + kBandDfMax + 1;
-    band_table_kernel<<<blocks_for(kBandDfMax + 1, 128), 128, 0, e->stream>>>(alpha, lo, hi, kBandDfMax);
+// Quantile tables at alpha +- band for 0 .. df degrees of freedom, kept while alpha stays and
+// grown in powers of two (a first call pays for the reach it needs).
+int ensure_quantiles(fpgm_engine *e, DevBuf &buf, double &have_alpha, int &have_df, double alpha, double band, int64_t df) {
+    if (have_alpha == alpha && buf.p && df <= have_df) return FPGM_OK;
+    int n = have_alpha == alpha ? std::max(have_df, 4096) : 4096;
+    while (n < df && n < kBandDfMax) n <<= 1;
+    if (have_alpha == alpha && buf.p && n <= have_df) return FPGM_OK;
+    have_alpha = -1.0;
+    RET(buf.ensure((size_t)2 * (n + 1) * sizeof(double)));
+    double *lo = buf.as<double>(), *hi = lo + n + 1;
+    band_table_kernel<<<blocks_for(2 * (n + 1), 64), 64, 0, e->stream>>>(alpha, band, lo, hi, n);
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(e->stream));
-    e->band_alpha = alpha;
+    have_alpha = alpha;
+    have_df = n;
     return FPGM_OK;
+}
+
+// Band-edge tables of the FP32 statistic.
+int ensure_band(fpgm_engine *e, double alpha, int64_t df = kBandDfMax) {
+    return ensure_quantiles(e, e->band, e->band_alpha, e->band_df, alpha, kBand, df);
 }
 
 // Largest table + marginals a level-d test can need, from the largest cardinality m.
@@ -1018,6 +1054,80 @@ int live_setup(fpgm_engine *e, int d) {
     return FPGM_OK;
 }
 
+void launch_warp_tier(fpgm_engine *e, const WaveArgs &a);
+
+// F for the samples of the engine's datasets, kept until a larger one comes.
+int fixed_setup(fpgm_engine *e) {
+    if (e->S > kFixedMaxSamples || e->fixed_n >= e->S) return FPGM_OK;
+    e->fixed_n = 0;
+    RET(e->fixed_f.ensure((size_t)(e->S + 1) * 8));
+    const double top = (double)e->S * log((double)std::max<int64_t>(e->S, 3));
+    const int k = 59 - (int)ceil(log2(top));  // four sums of at most `top` stay below 2^61
+    fixed_table_kernel<<<blocks_for(e->S + 1, 256), 256, 0, e->stream>>>(e->fixed_f.as<long long>(), e->S, ldexp(1.0, k));
+    CK(cudaGetLastError());
+    e->fixed_unit = ldexp(1.0, -k);
+    e->fixed_n = e->S;
+    return FPGM_OK;
+}
+
+// ---- tables per variable set (sets.cuh)
+// Level d's sets: an empty key table and the pool of tables, sized by what the level can need at
+// most while that is little, else by its edges (and grown when the level before ran out).  No
+// room: every test counts its own table.
+constexpr size_t kSetPoolMax = (size_t)4 << 30;
+int sets_setup(fpgm_engine *e, int d, int64_t n_active) {
+    e->sets_level = false;
+    if (!e->sets_on || e->fixed_n < e->S || d < 1 || e->wave_log || e->phase_timers.p) return FPGM_OK;
+    const int64_t tests = std::min<int64_t>(e->level_tests, 64 * n_active);
+    int32_t cap = 1 << 12;
+    while (cap < 4 * tests && cap < (1 << 22)) cap <<= 1;
+    const int64_t table = std::min<int64_t>(max_table_ints(e->h_card, d), kCtaInts);
+    const double most = 4.0 * (double)e->level_tests * (double)((table + 3) & ~(int64_t)3);
+    size_t pool = std::max<size_t>(e->sets_used * 4, (size_t)std::min(most, std::max(256.0 * cap, 6.4e7)));
+    pool = std::min(kSetPoolMax, std::max<size_t>(pool, (size_t)1 << 20));
+    if (e->set_pool_fixed) pool = e->set_pool_fixed;
+    if (e->set_tab.ensure((size_t)cap * 20 + 16) != FPGM_OK ||
+        (e->set_pool.bytes < pool && (e->set_pool.release(), e->set_pool.ensure(pool) != FPGM_OK)))
+        return FPGM_OK;
+    CK(cudaMemsetAsync(e->set_tab.p, 0, 16 + (size_t)cap * 8, e->stream));  // ints used, keys
+    e->sets_cap = cap;
+    e->sets_level = true;
+    // every set's keys fit (1 + |Z| / 2 entries, in half the table), every table, and no test's
+    // scratch passes a CTA's shared memory: then the kernels that count test by test stay out
+    e->sets_all = e->level_tests * (1 + d / 2) <= cap / 2 && most <= (double)e->set_pool.bytes &&
+                  2 * max_table_ints(e->h_card, d) <= kCtaInts;
+    return FPGM_OK;
+}
+
+// The set kernels of one wave on the current stream.  Returns launches issued.
+int launch_sets(fpgm_engine *e, const WaveArgs &a) {
+    const int grid = e->warp_small ? e->warp_blocks_small : e->ci_blocks;
+    const size_t smem = (size_t)kWarps * a.warp_ints * 4;
+    const bool cta = max_table_ints(e->h_card, a.d) * 2 > a.warp_ints;  // (offsets and scratch included)
+    if (e->warp_small)
+        set_count_warp_kernel<kWarpIntsSmall, 3><<<grid, kThreads, smem, e->stream>>>(a);
+    else
+        set_count_warp_kernel<kWarpInts, 2><<<grid, kThreads, smem, e->stream>>>(a);
+    set_count_cta_kernel<<<e->ci_blocks, kThreads, kSmemBytes, e->stream>>>(a);
+    if (e->warp_small)
+        set_score_warp_kernel<kWarpIntsSmall, 3><<<grid, kThreads, smem, e->stream>>>(a);
+    else
+        set_score_warp_kernel<kWarpInts, 2><<<grid, kThreads, smem, e->stream>>>(a);
+    if (cta) set_score_cta_kernel<<<e->ci_blocks, kThreads, kSmemBytes, e->stream>>>(a);
+    return 3 + cta;
+}
+
+// The tiers of a wave whose tables fit shared memory: from their sets' tables, and one by one
+// what found no room there.  Returns launches issued.
+int launch_shared_tiers(fpgm_engine *e, const WaveArgs &a) {
+    int n = 0;
+    if (a.sets.key) n += launch_sets(e, a);
+    if (a.sets.key && e->sets_all) return n;
+    launch_warp_tier(e, a);
+    ci_cta_kernel<<<e->ci_blocks, kThreads, kSmemBytes, e->stream>>>(a);
+    return n + 2;
+}
+
 // ---- shared strata (strata.cuh)
 // Tables: keys of nodes and pairs, then their fields; all sized by the two capacities.
 constexpr int kStrataNodes = 1 << 19, kStrataPairs = 1 << 20, kStrataBuild = 1 << 17;
@@ -1050,11 +1160,6 @@ void strata_args(fpgm_engine *e, StrataArgs &s) {
     s.pair_list = s.build_list + (size_t)(kStrataMaxSets + 1) * kStrataBuild;
     s.pair_list_cap = kStrataPairs;
     s.item_ref = e->strata_refs.as<int4>();
-    s.f = e->strata_f.as<long long>();
-    s.unit = e->strata_unit;
-    // 2 S counts of two or more at most over the four sums, half a unit each, doubled; and the
-    // FP64 rounding of the largest F
-    s.err = 2.0 * e->strata_unit + 1e-14;
 }
 
 // Level d's waves count through shared strata when a test can go past shared memory: buffers
@@ -1062,7 +1167,7 @@ void strata_args(fpgm_engine *e, StrataArgs &s) {
 int strata_setup(fpgm_engine *e, int d, bool first) {
     e->strata_level = false;
     if (first) e->strata_ready = false;
-    if (!e->strata_on || !e->wide_on || e->wave_log || e->phase_timers.p || e->S > kStrataMaxSamples || d < 1 ||
+    if (!e->strata_on || !e->wide_on || e->wave_log || e->phase_timers.p || e->fixed_n < e->S || d < 1 ||
         d + 1 > kStrataMaxSets || max_table_ints(e->h_card, d) <= kCtaInts - 64)
         return FPGM_OK;
     const size_t tab = kStrataKeyBytes + (size_t)kStrataNodes * 24 + (size_t)kStrataPairs * 16;
@@ -1076,7 +1181,9 @@ int strata_setup(fpgm_engine *e, int d, bool first) {
     const size_t least = std::max<size_t>((size_t)256 << 20, slot * 8192);
     size_t want = std::max(least, e->strata_pool.bytes);
     if (e->strata_ready && used[0] > e->strata_pool.bytes / 2) want = std::max(want, 4 * e->strata_pool.bytes);
-    if (want > e->strata_pool.bytes) {
+    if (e->strata_pool_fixed) {
+        if (!e->strata_pool.p) RET(e->strata_pool.ensure(e->strata_pool_fixed));
+    } else if (want > e->strata_pool.bytes) {
         size_t free_b = 0, total_b = 0;
         CK(cudaMemGetInfo(&free_b, &total_b));
         want = std::min(want, std::max(least, (size_t)std::min(32.0e9, 0.25 * (double)(free_b + e->strata_pool.bytes))));
@@ -1095,17 +1202,6 @@ int strata_setup(fpgm_engine *e, int d, bool first) {
         e->strata_used.ensure(64 + sizeof(StrataCounters)) != FPGM_OK) {
         e->strata_on = false;
         return FPGM_OK;
-    }
-    if (e->strata_f_n < e->S) {
-        RET(e->strata_f.ensure((size_t)(e->S + 1) * 8));
-        const double top = (double)e->S * log((double)std::max<int64_t>(e->S, 3));
-        const int k = 59 - (int)ceil(log2(top));  // four sums of at most `top` stay below 2^61
-        e->strata_unit = ldexp(1.0, -k);
-        strata_f_kernel<<<blocks_for(e->S + 1, 256), 256, 0, e->stream>>>(e->strata_f.as<long long>(), e->S,
-                                                                         ldexp(1.0, k));
-        CK(cudaGetLastError());
-        e->strata_f_n = e->S;
-        empty = true;  // sums of another unit
     }
     if (empty) {
         CK(cudaMemsetAsync(e->strata_tab.p, 0, kStrataKeyBytes, e->stream));
@@ -1139,10 +1235,23 @@ int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t ite
     a.counters = e->counters.as<int32_t>();
     a.stats = e->stats.as<unsigned long long>();
     a.alpha = alpha;
-    RET(ensure_band(e, alpha));
-    a.bt.lo = e->band.as<double>();
-    a.bt.hi = a.bt.lo + kBandDfMax + 1;
-    a.bt.dfmax = kBandDfMax;
+    const int64_t df = max_table_ints(e->h_card, d);  // a test's degrees of freedom are below its table's size
+    // the FP32 statistic's tables, unless every test of the wave is decided in fixed point
+    const bool gram = d == 0 && e->n_jobs == 1 && e->gram_on && e->gram_planned && e->gram_ok;
+    if (!(e->in_skeleton && e->fixed_n >= e->S && (gram || (d >= 1 && e->sets_level && e->sets_all)))) {
+        RET(ensure_band(e, alpha, df));
+        a.bt.lo = e->band.as<double>();
+        a.bt.hi = a.bt.lo + e->band_df + 1;
+        a.bt.dfmax = e->band_df;
+    }
+    if (e->in_skeleton && e->fixed_n >= e->S) {
+        RET(ensure_quantiles(e, e->tight, e->tight_alpha, e->tight_df, alpha, kTight, df));
+        a.fx.f = e->fixed_f.as<long long>();
+        a.fx.unit = e->fixed_unit;
+        a.fx.lo = e->tight.as<double>();
+        a.fx.hi = a.fx.lo + e->tight_df + 1;
+        a.fx.dfmax = e->tight_df;
+    }
     RET(e->item_vars.ensure((size_t)std::max<int64_t>(items, 1) * (2 + d) * 2 + 16));
     RET(e->lists.ensure((size_t)7 * std::max<int64_t>(items, 1) * 4 + 16));
     RET(e->flag.ensure((size_t)std::max<int64_t>(items, 1) + 16));
@@ -1185,6 +1294,21 @@ int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t ite
                 a.bm_prev_tab_cap = e->live_tab_cap;
             }
         }
+    }
+    if (e->sets_level && d >= 1) {
+        const size_t ni = (size_t)std::max<int64_t>(items, 1);
+        RET(e->set_items.ensure(ni * 2 * sizeof(int2)));
+        a.sets.used = e->set_tab.as<unsigned long long>();
+        a.sets.key = reinterpret_cast<uint64_t *>(e->set_tab.as<char>() + 16);
+        a.sets.cap = e->sets_cap;
+        a.sets.probe = e->sets_all ? e->sets_cap : kEnterProbe;
+        a.sets.h = reinterpret_cast<long long *>(a.sets.key + e->sets_cap);
+        a.sets.off = reinterpret_cast<int32_t *>(a.sets.h + e->sets_cap);
+        a.sets.pool = e->set_pool.as<int32_t>();
+        a.sets.pool_cap = e->set_pool.bytes / 4;
+        a.sets.items = e->set_items.as<int2>();
+        a.sets.fresh = a.sets.items + ni;
+        a.sets.few = e->ci_blocks;
     }
     if (e->strata_level && d >= 1) {
         RET(e->strata_refs.ensure((size_t)std::max<int64_t>(items, 1) * sizeof(int4)));
@@ -1238,7 +1362,8 @@ int launch_tiers(fpgm_engine *e, const WaveArgs &a) {
 int run_waves_graph(fpgm_engine *e, double alpha, int d, int64_t n_active, fpgm_pc_stats *st, int level_idx,
                     const WaveArgs &proto) {
     unsigned long long *dstat = e->stats.as<unsigned long long>();
-    const int64_t cap = std::max<int64_t>(n_active, kMaxItems);  // items of one wave at most
+    // items of one wave at most
+    const int64_t cap = std::max<int64_t>(n_active, std::min<int64_t>(kMaxItems, std::max<int64_t>(e->level_tests, 1 << 16)));
     WaveArgs a = proto;
     RET(wave_args_base(e, a, alpha, d, cap));
     a.adjl = proto.adjl;
@@ -1292,10 +1417,8 @@ int run_waves_graph(fpgm_engine *e, double alpha, int d, int64_t n_active, fpgm_
                                       (int)(n_active + 1), e->stream);
         wave_stamp_kernel<<<1, 1, 0, e->stream>>>(ctl, -1);
         classify_kernel<SRC_WAVE><<<e->ci_blocks, kThreads, 0, e->stream>>>(a);
-        launch_warp_tier(e, a);
-        ci_cta_kernel<<<e->ci_blocks, kThreads, kSmemBytes, e->stream>>>(a);
+        per_wave = 8 + launch_shared_tiers(e, a);  // prep, plan, 3 stamps, classify, reduce, tail (+ tier 2)
         wave_stamp_kernel<<<1, 1, 0, e->stream>>>(ctl, 0);
-        per_wave = 9;  // prep, plan, 3 stamps, classify, warp tier, CTA tier, reduce, tail (+ tier 2)
         if (a.strata_card) per_wave += launch_strata(e, a);
         if (a.slot_mem) per_wave += launch_compact(e, a, e->n_slots);
         wave_stamp_kernel<<<1, 1, 0, e->stream>>>(ctl, 1);
@@ -1379,7 +1502,7 @@ int run_waves_and_count(fpgm_engine *e, double alpha, int d, int64_t n_active, f
         size_t sb = e->scan_tmp.bytes;
         CK(cub::DeviceScan::ExclusiveSum(e->scan_tmp.p, sb, e->g.as<int32_t>(), e->off.as<int32_t>(),
                                          (int)(n_active + 1), e->stream));
-        CK(cudaMemsetAsync(e->counters.p, 0, 64, e->stream));
+        CK(cudaMemsetAsync(e->counters.p, 0, kCounterBytes, e->stream));
         CK(cudaMemsetAsync(dstat + ST_BYTES_SHARED, 0, 16, e->stream));  // this wave's bytes
         a.off = e->off.as<int32_t>();
         a.n_edges = (int32_t)n_active;
@@ -1394,10 +1517,8 @@ int run_waves_and_count(fpgm_engine *e, double alpha, int d, int64_t n_active, f
             st->kernel_launches += nl + 3;  // plan, one-hot + GEMM, scoring, reduce
         } else {
             classify_kernel<SRC_WAVE><<<e->ci_blocks, kThreads, 0, e->stream>>>(a);
-            launch_warp_tier(e, a);
-            ci_cta_kernel<<<e->ci_blocks, kThreads, kSmemBytes, e->stream>>>(a);
+            st->kernel_launches += 3 + launch_shared_tiers(e, a);  // plan, classify, reduce
             CK(cudaGetLastError());
-            st->kernel_launches += 5;  // plan, classify, warp tier, CTA tier, reduce
         }
         CK(cudaEventRecord(e->ev1, e->stream));
         a.dbg = e->phase_timers.as<unsigned long long>();
@@ -1503,11 +1624,13 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
         }
         ~LiveScope() {
             e->live_level[0] = e->live_level[1] = -1;
-            e->strata_level = false;
+            e->strata_level = e->sets_level = e->in_skeleton = false;
             e->live_write = false;
             e->live_in_skeleton = false;
         }
     } live_scope(e);
+    e->in_skeleton = true;
+    RET(fixed_setup(e));
     if (e->live_on) {  // contributing-sample counts, measured level by level
         RET(e->live_stat.ensure(16));
         CK(cudaMemsetAsync(e->live_stat.p, 0, 16, e->stream));
@@ -1622,6 +1745,12 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
                 gram = e->gram_ok;
             }
             if (!gram) RET(live_setup(e, d));
+            {  // a test per rank: at most C(max_deg - 1, d) from either side of an edge
+                double c = 2.0 * (double)n_active;
+                for (int k = 0; k < d; ++k) c = std::min(1e15, c * std::max(0, max_deg - 1 - k) / (k + 1));
+                e->level_tests = d == 0 ? n_active : (int64_t)c + 64;
+            }
+            RET(sets_setup(e, d, n_active));
             RET(strata_setup(e, d, d <= 1));
             RET(run_waves_and_count(e, alpha, d, n_active, st, st->n_levels, a, gram));
             if (e->live_on && e->live_stat.p) {
@@ -1659,9 +1788,11 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
         degree_kernel<<<blocks_for(n, 128), 128, 0, e->stream>>>(e->bits.as<uint32_t>(), n, W, dstat);
         CK(cudaGetLastError());
         st->kernel_launches += 1;
-        unsigned long long hs[ST_COUNT];
+        unsigned long long hs[ST_COUNT], h_sets_used = 0;
         CK(cudaMemcpyAsync(hs, dstat, sizeof hs, cudaMemcpyDeviceToHost, e->stream));
+        if (e->sets_level) CK(cudaMemcpyAsync(&h_sets_used, e->set_tab.p, 8, cudaMemcpyDeviceToHost, e->stream));
         CK(cudaStreamSynchronize(e->stream));
+        e->sets_used = h_sets_used;
         const int64_t removed = (int64_t)hs[ST_REMOVED];
         log_count += removed;
         var_count += removed * d;
@@ -1773,12 +1904,12 @@ int plain_test(fpgm_engine *e, int x, int y, const int *z, int d, double alpha, 
         CK(cudaMemsetAsync(e->plain_ws.p, 0, e->plain_ws.bytes, e->stream));
     }
     RET(e->detail_buf.ensure(sizeof(fpgm_ci_result) * 64));
-    RET(ensure_band(e, alpha));
     // table size decides: dense grid-wide kernel, or the compact-strata kernel on one CTA
     double cells = (double)e->h_card[x] * e->h_card[y], dz = 1.0;
     for (int k = 0; k < d; ++k) dz *= e->h_card[z[k]];
     cells *= dz;
     const double need = cells + dz * (e->h_card[x] + e->h_card[y] + 1);
+    RET(ensure_band(e, alpha, (int64_t)std::min(cells, (double)kBandDfMax)));
     if (need <= (double)kPlainInts) {
         PlainArgs p;
         memset(&p, 0, sizeof p);
@@ -1792,8 +1923,8 @@ int plain_test(fpgm_engine *e, int x, int y, const int *z, int d, double alpha, 
         for (int k = 0; k < d + 2; ++k) p.col_off[k] = e->h_var_off[p.vars[k]];
         p.alpha = alpha;
         p.bt.lo = e->band.as<double>();
-        p.bt.hi = p.bt.lo + kBandDfMax + 1;
-        p.bt.dfmax = kBandDfMax;
+        p.bt.hi = p.bt.lo + e->band_df + 1;
+        p.bt.dfmax = e->band_df;
         p.want_hash = want_hash;
         p.gtab = e->plain_ws.as<int32_t>();
         p.done = reinterpret_cast<int32_t *>(e->plain_ws.as<char>() + (size_t)kPlainInts * 4);
@@ -2133,7 +2264,7 @@ extern "C" int fpgm_ci_test_batch(fpgm_engine *e, const int32_t *tests, int32_t 
     RET(e->tests_buf.ensure((size_t)n_tests * (2 + d) * 4));
     RET(e->detail_buf.ensure((size_t)n_tests * sizeof(fpgm_ci_result)));
     CK(cudaMemcpyAsync(e->tests_buf.p, tests, (size_t)n_tests * (2 + d) * 4, cudaMemcpyHostToDevice, e->stream));
-    CK(cudaMemsetAsync(e->counters.p, 0, 64, e->stream));
+    CK(cudaMemsetAsync(e->counters.p, 0, kCounterBytes, e->stream));
     CK(cudaMemsetAsync(e->stats.p, 0, ST_COUNT * 8, e->stream));
     WaveArgs a;
     RET(wave_args_base(e, a, alpha, d, n_tests));

@@ -26,9 +26,7 @@
 // Nodes and pairs live until the skeleton ends: the sets Z + o of level d are the sets Z of
 // level d + 1, and the pairs (Z + o, c) its pairs (Z, c).
 //
-// F is held as a 64-bit integer, round(n ln n 2^k) with k as large as the sample count allows,
-// so the sums are exact and in any order the same; the statistic's error is at most half a unit
-// per count (StrataArgs::err), below 1e-6 at 100,000 samples.
+// F is the fixed-point table of fixed.cuh: exact sums, whatever their order.
 #pragma once
 #include "ci_kernels.cuh"
 
@@ -39,8 +37,6 @@ constexpr int kStrataInts = 27 * 1024;               // 108 KB of shared counter
 constexpr uint32_t kNoStratum = 0xffffu;
 constexpr int kStrataMaxSets = kMaxCond + 2;         // sizes of built sets: 1 .. |Z| + 1
 constexpr int kStrataMaxCard = 32;                   // states of the test's o (one mask word)
-constexpr int64_t kStrataMaxSamples = (int64_t)1 << 20;  // beyond: the fixed-point error bound grows too large
-constexpr int kStrataProbe = 128;
 
 // counters, cleared for every wave: nodes to build per size, taken per size, pairs, tests
 struct StrataCounters {
@@ -66,26 +62,7 @@ struct StrataArgs {
     int32_t build_cap, pair_list_cap;
     int4 *item_ref;        // per listed test: nodes Z and Z + o, pairs (Z, c) and (Z + o, c)
     StrataCounters *sc;
-    const long long *f;    // F
-    double unit;           // G^2 = 2 unit x (sum of F's)
-    double err;            // error bound of the statistic per sample
 };
-
-__device__ inline int strata_enter(uint64_t *keys, int cap, uint64_t key, bool *fresh) {
-    uint32_t h = (uint32_t)((key * 0x9E3779B97F4A7C15ull) >> 32) & (uint32_t)(cap - 1);
-    *fresh = false;
-    for (int p = 0; p < kStrataProbe; ++p) {
-        uint64_t k = *(volatile uint64_t *)&keys[h];
-        if (k == key) return (int)h;
-        if (k == 0) {
-            k = key_cas(&keys[h], 0ull, key);
-            if (k == 0) *fresh = true;
-            if (k == 0 || k == key) return (int)h;
-        }
-        h = (h + 1) & (uint32_t)(cap - 1);
-    }
-    return -1;
-}
 
 // The trie node of a set of m ascending variables (entered with every prefix that is missing);
 // -1 when there is no room.
@@ -93,7 +70,7 @@ __device__ inline int strata_node(const StrataArgs &s, const uint16_t *v, int m)
     int at = -1;
     for (int i = 0; i < m; ++i) {
         bool fresh;
-        at = strata_enter(s.node_key, s.node_cap, ((uint64_t)(at + 1) << 16 | v[i]) | (1ull << 62), &fresh);
+        at = table_enter(s.node_key, s.node_cap, kEnterProbe, ((uint64_t)(at + 1) << 16 | v[i]) | (1ull << 62), &fresh);
         if (at < 0) return -1;
         if (fresh) {
             s.node_n[at] = -1;
@@ -107,7 +84,7 @@ __device__ inline int strata_node(const StrataArgs &s, const uint16_t *v, int m)
 
 __device__ inline int strata_pair_of(const StrataArgs &s, int node, int v) {
     bool fresh;
-    const int at = strata_enter(s.pair_key, s.pair_cap, ((uint64_t)node << 16 | (uint64_t)v) | (1ull << 62), &fresh);
+    const int at = table_enter(s.pair_key, s.pair_cap, kEnterProbe, ((uint64_t)node << 16 | (uint64_t)v) | (1ull << 62), &fresh);
     if (fresh) {
         s.pair_a[at] = -1;
         atomicAdd(&s.pool_used[2], 1ull);
@@ -263,7 +240,7 @@ __global__ void __launch_bounds__(kStrataThreads, 2) strata_count_kernel(WaveArg
                         ++met;
                         if (m >= 2) {
                             ++kept;
-                            h += __ldg(&s.f[m]);
+                            h += __ldg(&a.fx.f[m]);
                             big = max(big, m);
                         }
                     }
@@ -394,21 +371,22 @@ __global__ void __launch_bounds__(kStrataThreads, 2) strata_test_kernel(WaveArgs
             int dec = -1;
             if (ok) {
                 const long long hs = s.pair_h[r.w] - s.pair_h[r.z] - s.node_h[r.y] + s.node_h[r.x];
-                const double g2 = 2.0 * s.unit * (double)hs;
-                const double err = s.err * (double)a.var_S[a.item_vars[(int64_t)item * (d + 2) + d]];
-                dec = df == 0 ? 1 : band_decide(df, g2, err, a.bt);
-                if (dec < 0 && df > a.bt.dfmax) {
-                    const double pw = chisq_pvalue_wh(g2, (double)df);
-                    const double slack = kBand + kWhMargin + 2.0 * err * 0.3 / sqrt((double)df);
-                    if (fabs(pw - a.alpha) > slack) dec = pw > a.alpha;
-                }
-                if (dec < 0) {  // within 1e-3 of alpha: the p-value itself, unless its error bound reaches alpha
-                    const double p = chisq_pvalue(fmax(g2, 0.0), df);
-                    // the density of a chi-square is at most 1/2 past two degrees of freedom; at one it is
-                    // below 0.45 wherever p is near an alpha of at most 0.3
-                    const double slack = 1e-7 + err;
-                    if (fabs(p - a.alpha) > slack && (df > 1 || g2 > 1.0)) dec = p > a.alpha;
-                    if (dec >= 0 && tid == 0) atomicAdd(&a.stats[ST_RECHECK], 1ull);
+                const int64_t S = a.var_S[a.item_vars[(int64_t)item * (d + 2) + d]];
+                // the four sums hold at most 2 S counts of two or more
+                double g2;
+                dec = fixed_decide(a.fx, df, hs, 2 * S, S, &g2);
+                if (dec < 0) {
+                    const double err = 2.0 * a.fx.unit * (double)S + 2e-14 * (double)S;
+                    if (df > a.fx.dfmax) {
+                        const double pw = chisq_pvalue_wh(g2, (double)df);
+                        const double slack = kBand + kWhMargin + 2.0 * err * 0.3 / sqrt((double)df);
+                        if (fabs(pw - a.alpha) > slack) dec = pw > a.alpha;
+                    }
+                    if (dec < 0) {  // the p-value, unless its error bound (a density of at most 1/2) reaches alpha
+                        const double p = chisq_pvalue(fmax(g2, 0.0), df);
+                        if (fabs(p - a.alpha) > 1e-7 + err && (df > 1 || g2 > 1.0)) dec = p > a.alpha;
+                        if (dec >= 0 && tid == 0) atomicAdd(&a.stats[ST_RECHECK], 1ull);
+                    }
                 }
             }
             if (tid == 0) {
@@ -423,12 +401,6 @@ __global__ void __launch_bounds__(kStrataThreads, 2) strata_test_kernel(WaveArgs
         }
         __syncthreads();
     }
-}
-
-// F(n) = n ln n in units of 2^-k
-__global__ void strata_f_kernel(long long *f, int64_t n_max, double scale) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i <= n_max) f[i] = i < 2 ? 0 : __double2ll_rn((double)i * log((double)i) * scale);
 }
 
 }  // namespace fpgm
