@@ -29,11 +29,12 @@ namespace fpgm {
 // compact kernel's global hash (lists 3-4 and 5 of WaveArgs::lists)
 // C_WIDET / C_WIDEQ / C_WIDEW: tests published for partition-parallel scoring, the
 // (test, partition) items queued for it, and the items taken
-// C_SETW / C_SETC: variable sets to count by a warp / a CTA, C_SCOREW / C_SCOREC: tests to score
-// from their set's table by a warp / a CTA, and the ones taken (sets.cuh)
+// C_SET + k: variable sets to count by 2^k warps (k = 4: a CTA of set_count_big_kernel),
+// C_SCOREW / C_SCOREC: tests to score from their set's table by a warp / a CTA, and the ones
+// taken of each (sets.cuh)
 // C_STRATA: tests counted through their shared variable sets (strata.cuh; list 6)
 enum { C_TIER0 = 0, C_TIER1, C_TIER2, C_WORK0, C_WORK1, C_WORK2, C_PART, C_WORKP, C_RETRY, C_WORKR, C_WIDET, C_WIDEQ,
-       C_WIDEW, C_STRATA, C_SETW, C_WSETW, C_SETC, C_WSETC, C_SCOREW, C_WSCOREW, C_SCOREC, C_WSCOREC, C_COUNT };
+       C_WIDEW, C_STRATA, C_SET, C_WSET = C_SET + 5, C_SCOREW = C_WSET + 5, C_WSCOREW, C_SCOREC, C_WSCOREC, C_COUNT };
 constexpr int kCounterBytes = 128;
 static_assert(C_COUNT * 4 <= kCounterBytes, "counters are cleared together");
 // stats[] slots (unsigned long long)
@@ -132,9 +133,9 @@ struct SetArgs {
     int32_t *pool;
     unsigned long long pool_cap;
     unsigned long long *used;  // ints of the pool handed out
-    int2 *fresh;               // sets to count (entry, an item): a warp's from the front, a CTA's from the end
-    int2 *items;               // tests to score (entry, item), likewise
-    int32_t few;               // at most this many new sets: each is counted by a CTA
+    int2 *fresh;               // sets to count (entry, an item): five lists of list_cap
+    int2 *items;               // tests to score (entry, item): a warp's from the front, a CTA's from the end
+    int32_t few;               // at most this many new sets: each is counted by a whole CTA
 };
 
 struct WaveArgs {
@@ -316,6 +317,26 @@ __device__ inline int table_enter(uint64_t *keys, int cap, int probe, uint64_t k
     return -1;
 }
 
+// Replicas (log2) a set's table is counted in, and how many warps (log2) share them.  Every lane
+// of a warp counts into a copy of its own while the table allows it, because the shared-memory
+// atomics are what bounds a count (one conflict-free warp instruction a clock): with one warp
+// per table of 8 KB they spent 31% (43 cells on average) to 60% (150) of their cycles on bank
+// conflicts.  So larger tables get more warps, whose copies they share; and a table is not
+// copied so often that clearing and summing the copies would cost more than the samples.
+constexpr int kSetWarpInts = 2048;  // per warp of set_count_kernel
+__host__ __device__ inline int set_replicas(int cells, int64_t S, int ints) {
+    int l = 0;
+    while (l < 5 && (cells << (l + 1)) <= ints && ((int64_t)cells << (l + 3)) <= S) ++l;
+    return l;
+}
+__host__ __device__ inline int set_class(int cells, int64_t S) {
+    if (cells > 8 * kSetWarpInts) return 4;
+    const int want = set_replicas(cells, S, 8 * kSetWarpInts);
+    int k = 0;
+    while (k < 3 && (cells << want) > (kSetWarpInts << k)) ++k;
+    return k;
+}
+
 // Entry of the set of m >= 3 ascending variables: the first three in one key, then two at a
 // time after the entry reached so far (the keys hold the variables themselves, so two sets
 // never share an entry).  -1: no room.
@@ -408,9 +429,9 @@ __global__ void classify_kernel(WaveArgs a) {
                     const bool room = o + cells <= a.sets.pool_cap;
                     a.sets.off[at] = room ? (int32_t)o : -1;
                     if (room) {
-                        const bool warp = cells <= a.warp_ints;
-                        const int q = atomicAdd(&a.counters[warp ? C_SETW : C_SETC], 1);
-                        a.sets.fresh[warp ? q : a.list_cap - 1 - q] = make_int2(at, item);
+                        const int k = set_class(cells, a.var_S[x]);
+                        const int q = atomicAdd(&a.counters[C_SET + k], 1);
+                        a.sets.fresh[k * a.list_cap + q] = make_int2(at, item);
                     }
                 }
                 const bool warp = work <= a.warp_ints;
@@ -466,37 +487,117 @@ __device__ __forceinline__ void horner_pair(uint32_t (&ca)[8], uint32_t (&cb)[8]
 }
 
 // Adds the samples of ncols columns (Horner order) to a table of 2^lgR replicas interleaved cell
-// by cell (cell c of replica r at c << lgR | r; this lane's is lane mod 2^lgR).  Called by
-// kStep threads, t = 0 .. kStep - 1.  Two samples share a 32-bit register until the end, where
-// one dot-product instruction takes a 16-bit code to its shared-memory address.
-template <int kStep>
-__device__ __forceinline__ void count_columns(int *rep, int lgR, int lane, const uint8_t *const *col,
-                                              const uint32_t *dim, int ncols, int64_t S, int t) {
-    const uint32_t base = (uint32_t)__cvta_generic_to_shared(rep + (lane & ((1 << lgR) - 1)));
-    const uint32_t mlo = 4u << lgR, mhi = mlo << 8;
-    const int64_t nvec = S >> 4;
-    auto add = [](uint32_t at) { asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(at) : "memory"); };
-    for (int64_t v = t; v < nvec; v += 2 * kStep) {
-        const bool two = v + kStep < nvec;
-        uint32_t ca[8], cb[8];
-        horner_pair(ca, cb, col, dim, ncols, v, v + kStep, two);
+// by cell (cell c of replica r at c << lgR | r; this lane's is lane mod 2^lgR).  Called by step
+// threads, t = 0 .. step - 1.  Codes are packed: four samples in the bytes of a register while
+// they stay below 256 (one multiply-add per column and four samples), then two in its halves;
+// one dot-product instruction takes a code from there to its shared-memory address.  Three
+// columns of up to 256 cells take 3.1 instructions per sample (8.4 with two samples per
+// register throughout and a shift and add per address).
+__device__ __forceinline__ void count_at(uint32_t at) { asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(at) : "memory"); }
+
+template <int N, bool kBytes>
+__device__ __forceinline__ void count_vector(const uint4 (&w)[N], const uint32_t (&m)[N], int nb, uint32_t base, uint32_t mul) {
+    uint32_t c[4] = {w[0].x, w[0].y, w[0].z, w[0].w};
+#pragma unroll
+    for (int j = 1; j < N; ++j)
+        if (kBytes || j < nb) {
+            c[0] = c[0] * m[j] + w[j].x;
+            c[1] = c[1] * m[j] + w[j].y;
+            c[2] = c[2] * m[j] + w[j].z;
+            c[3] = c[3] * m[j] + w[j].w;
+        }
+    if (kBytes) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) count_at(__dp4a(c[q], mul << (8 * b), base));
+    } else {
+        uint32_t h[8];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            h[2 * q] = __byte_perm(c[q], 0, 0x4140);
+            h[2 * q + 1] = __byte_perm(c[q], 0, 0x4342);
+        }
+#pragma unroll
+        for (int j = 1; j < N; ++j)
+            if (j >= nb) horner16(h, w[j], m[j]);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            add(__dp2a_lo(ca[q], mlo, base));
-            add(__dp2a_lo(ca[q], mhi, base));
+            count_at(__dp2a_lo(h[q], mul, base));
+            count_at(__dp2a_lo(h[q], mul << 8, base));
         }
-        if (two) {
+    }
+}
+
+template <int N, bool kBytes>
+__device__ __forceinline__ void count_vectors(const uint8_t *const *col, const uint32_t *dim, int nb, int64_t nvec, int t,
+                                              int step, uint32_t base, uint32_t mul) {
+    const uint4 *p[N];
+    uint32_t m[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        p[j] = reinterpret_cast<const uint4 *>(col[j]);
+        m[j] = dim[j];
+    }
+    const int n = (int)nvec;
+    int v = t;
+    for (; v + step < n; v += 2 * step) {  // two vectors' loads in flight
+        uint4 a[N], b[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            a[j] = __ldg(p[j] + v);
+            b[j] = __ldg(p[j] + v + step);
+        }
+        count_vector<N, kBytes>(a, m, nb, base, mul);
+        count_vector<N, kBytes>(b, m, nb, base, mul);
+    }
+    if (v < n) {
+        uint4 a[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) a[j] = __ldg(p[j] + v);
+        count_vector<N, kBytes>(a, m, nb, base, mul);
+    }
+}
+
+__device__ __forceinline__ void count_columns(int *rep, int lgR, int lane, const uint8_t *const *col,
+                                              const uint32_t *dim, int ncols, int64_t S, int t, int step) {
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(rep + (lane & ((1 << lgR) - 1)));
+    const uint32_t mul = 4u << lgR;
+    const int64_t nvec = S >> 4;
+    int nb = 1;  // leading columns whose codes fit a byte
+    for (uint32_t p = dim[0]; nb < ncols && p * dim[nb] <= 256u; ++nb) p *= dim[nb];
+    if (nb == ncols && ncols >= 2 && ncols <= 5) {
+        if (ncols == 2) count_vectors<2, true>(col, dim, nb, nvec, t, step, base, mul);
+        else if (ncols == 3) count_vectors<3, true>(col, dim, nb, nvec, t, step, base, mul);
+        else if (ncols == 4) count_vectors<4, true>(col, dim, nb, nvec, t, step, base, mul);
+        else count_vectors<5, true>(col, dim, nb, nvec, t, step, base, mul);
+    } else if (ncols >= 3 && ncols <= 5) {
+        if (ncols == 3) count_vectors<3, false>(col, dim, nb, nvec, t, step, base, mul);
+        else if (ncols == 4) count_vectors<4, false>(col, dim, nb, nvec, t, step, base, mul);
+        else count_vectors<5, false>(col, dim, nb, nvec, t, step, base, mul);
+    } else {
+        for (int64_t v = t; v < nvec; v += 2 * step) {
+            const bool two = v + step < nvec;
+            uint32_t ca[8], cb[8];
+            horner_pair(ca, cb, col, dim, ncols, v, v + step, two);
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-                add(__dp2a_lo(cb[q], mlo, base));
-                add(__dp2a_lo(cb[q], mhi, base));
+                count_at(__dp2a_lo(ca[q], mul, base));
+                count_at(__dp2a_lo(ca[q], mul << 8, base));
+            }
+            if (two) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    count_at(__dp2a_lo(cb[q], mul, base));
+                    count_at(__dp2a_lo(cb[q], mul << 8, base));
+                }
             }
         }
     }
-    for (int64_t s = (S & ~(int64_t)15) + t; s < S; s += kStep) {
+    for (int64_t s = (S & ~(int64_t)15) + t; s < S; s += step) {
         uint32_t c = 0;
         for (int j = 0; j < ncols; ++j) c = c * dim[j] + col[j][s];
-        add(base + (c << lgR << 2));
+        count_at(base + (c << lgR << 2));
     }
 }
 
@@ -568,7 +669,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) ci_warp_kernel(WaveArgs 
         __syncwarp();
         // with 32 replicas every lane owns one bank, so a warp's 32 increments never conflict
         // whatever cells they hit
-        count_columns<32>(rep, lgR, lane, s_col[warp], s_dim[warp], ncols, S, lane);
+        count_columns(rep, lgR, lane, s_col[warp], s_dim[warp], ncols, S, lane, 32);
         __syncwarp();
         if (R > 1) {
             for (int c = lane; c < (int)cells; c += 32) {
@@ -623,7 +724,7 @@ __global__ void __launch_bounds__(kThreads, 2) ci_cta_kernel(WaveArgs a) {
         int *ni = tab + cells, *nj = ni + dz * dx, *nk = nj + dz * dy;
         for (int i = tid; i < (cells << lgR); i += kThreads) rep[i] = 0;
         __syncthreads();
-        count_columns<kThreads>(rep, lgR, lane, s_col, s_dim, ncols, S, tid);
+        count_columns(rep, lgR, lane, s_col, s_dim, ncols, S, tid, kThreads);
         __syncthreads();
         if (R > 1) {
             for (int c = tid; c < cells; c += kThreads) {

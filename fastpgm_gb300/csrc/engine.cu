@@ -430,51 +430,56 @@ __global__ void wave_plan_kernel(int n_edges, const uint8_t *status, const uint6
     g[e] = v;
 }
 
+// One warp per edge: its ranks' results 32 at a time (an edge can have 4,096 in a wave).
 __global__ void wave_reduce_kernel(int n_edges, const int32_t *off, const uint8_t *flag, uint8_t *status,
                                    uint64_t *next, const uint64_t *total, uint64_t *seprank,
                                    unsigned long long *stats) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned long long bad = 0, exec = 0, det = 0, unresolved = 0;
-    if (e < n_edges) {
+    __shared__ unsigned long long s_sum[4];  // bad, executed, deterministic, unresolved
+    const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+    if (threadIdx.x < 4) s_sum[threadIdx.x] = 0;
+    __syncthreads();
+    unsigned long long bad = 0, exec = 0, det = 0, unresolved = 0;  // lane 0's
+    for (int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < n_edges; e += warps) {
         const int o = off[e], g = off[e + 1] - o;
-        if (g > 0) {
-            int first = -1;
-            for (int k = 0; k < g; ++k) {
-                const uint8_t f = flag[o + k];
-                if (f == 2) bad = 1;
-                if (f == 1) {
-                    first = k;
-                    break;
-                }
-            }
-            exec = (unsigned long long)g;
+        if (g <= 0) continue;
+        int first = -1;
+        for (int k0 = 0; k0 < g && first < 0; k0 += 32) {
+            const uint8_t f = k0 + lane < g ? flag[o + k0 + lane] : 0;
+            const unsigned hit = __ballot_sync(0xffffffffu, f == 1), odd = __ballot_sync(0xffffffffu, f == 2);
+            if (hit) first = k0 + __ffs(hit) - 1;
+            if (odd && (!hit || __ffs(odd) < __ffs(hit))) bad = 1;
+        }
+        if (lane == 0) {
+            exec += (unsigned long long)g;
             if (first >= 0) {
                 status[e] = kStatusRemoved;
                 seprank[e] = next[e] + first;
-                det = (unsigned long long)(first + 1);
+                det += (unsigned long long)(first + 1);
             } else {
                 const uint64_t nx = next[e] + g;
                 next[e] = nx;
-                det = (unsigned long long)g;
+                det += (unsigned long long)g;
                 if (nx == total[e]) status[e] = kStatusKept;
-                else unresolved = 1;
+                else ++unresolved;
             }
         }
     }
-    // one atomic per warp and counter: the level-0 wave has one edge per thread
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-        bad += __shfl_xor_sync(0xffffffffu, bad, s);
-        exec += __shfl_xor_sync(0xffffffffu, exec, s);
-        det += __shfl_xor_sync(0xffffffffu, det, s);
-        unresolved += __shfl_xor_sync(0xffffffffu, unresolved, s);
+    if (lane == 0) {
+        if (bad) atomicAdd(&s_sum[0], bad);
+        if (exec) atomicAdd(&s_sum[1], exec);
+        if (det) atomicAdd(&s_sum[2], det);
+        if (unresolved) atomicAdd(&s_sum[3], unresolved);
     }
-    if ((threadIdx.x & 31) == 0) {
-        if (bad) atomicAdd(&stats[ST_UNSUPPORTED], bad);
-        if (exec) atomicAdd(&stats[ST_EXEC], exec);
-        if (det) atomicAdd(&stats[ST_DET], det);
-        if (unresolved) atomicAdd(&stats[ST_UNRESOLVED], unresolved);
-    }
+    __syncthreads();
+    if (threadIdx.x < 4 && s_sum[threadIdx.x])
+        atomicAdd(&stats[threadIdx.x == 0   ? ST_UNSUPPORTED
+                         : threadIdx.x == 1 ? ST_EXEC
+                         : threadIdx.x == 2 ? ST_DET
+                                            : ST_UNRESOLVED],
+                  s_sum[threadIdx.x]);
+}
+inline int reduce_blocks(int64_t n_edges, int num_sms) {
+    return (int)std::min<int64_t>((n_edges + 7) / 8, 8 * (int64_t)num_sms);
 }
 
 // apply removals, log (pair, sepset) -- sepset rebuilt from its rank
@@ -741,13 +746,11 @@ extern "C" int fpgm_engine_create(int32_t device, fpgm_engine **out) {
     CK(cudaFuncSetAttribute(level0_gram_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     CK(cudaFuncSetAttribute(strata_count_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStrataInts * 4));
     CK(cudaFuncSetAttribute(strata_count_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStrataInts * 4));
-    CK(cudaFuncSetAttribute(set_count_warp_kernel<kWarpInts, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    CK(cudaFuncSetAttribute(set_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWarps * kSetWarpInts * 4));
     CK(cudaFuncSetAttribute(set_score_warp_kernel<kWarpInts, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    CK(cudaFuncSetAttribute(set_count_warp_kernel<kWarpIntsSmall, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            kWarps * kWarpIntsSmall * 4));
     CK(cudaFuncSetAttribute(set_score_warp_kernel<kWarpIntsSmall, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             kWarps * kWarpIntsSmall * 4));
-    CK(cudaFuncSetAttribute(set_count_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    CK(cudaFuncSetAttribute(set_count_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     CK(cudaFuncSetAttribute(set_score_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     CK(cudaFuncSetAttribute(strata_test_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStrataInts * 4));
     CK(cudaFuncSetAttribute(ci_plain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
@@ -1103,18 +1106,16 @@ int sets_setup(fpgm_engine *e, int d, int64_t n_active) {
 int launch_sets(fpgm_engine *e, const WaveArgs &a) {
     const int grid = e->warp_small ? e->warp_blocks_small : e->ci_blocks;
     const size_t smem = (size_t)kWarps * a.warp_ints * 4;
-    const bool cta = max_table_ints(e->h_card, a.d) * 2 > a.warp_ints;  // (offsets and scratch included)
-    if (e->warp_small)
-        set_count_warp_kernel<kWarpIntsSmall, 3><<<grid, kThreads, smem, e->stream>>>(a);
-    else
-        set_count_warp_kernel<kWarpInts, 2><<<grid, kThreads, smem, e->stream>>>(a);
-    set_count_cta_kernel<<<e->ci_blocks, kThreads, kSmemBytes, e->stream>>>(a);
+    const int64_t most = max_table_ints(e->h_card, a.d);
+    const bool big = most > 8 * kSetWarpInts, cta = 2 * most > a.warp_ints;  // (offsets and scratch included)
+    set_count_kernel<<<3 * e->num_sms, kThreads, kWarps * kSetWarpInts * 4, e->stream>>>(a);
+    if (big) set_count_big_kernel<<<e->ci_blocks, kThreads, kSmemBytes, e->stream>>>(a);
     if (e->warp_small)
         set_score_warp_kernel<kWarpIntsSmall, 3><<<grid, kThreads, smem, e->stream>>>(a);
     else
         set_score_warp_kernel<kWarpInts, 2><<<grid, kThreads, smem, e->stream>>>(a);
     if (cta) set_score_cta_kernel<<<e->ci_blocks, kThreads, kSmemBytes, e->stream>>>(a);
-    return 3 + cta;
+    return 2 + big + cta;
 }
 
 // The tiers of a wave whose tables fit shared memory: from their sets' tables, and one by one
@@ -1297,7 +1298,7 @@ int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t ite
     }
     if (e->sets_level && d >= 1) {
         const size_t ni = (size_t)std::max<int64_t>(items, 1);
-        RET(e->set_items.ensure(ni * 2 * sizeof(int2)));
+        RET(e->set_items.ensure(ni * 6 * sizeof(int2)));
         a.sets.used = e->set_tab.as<unsigned long long>();
         a.sets.key = reinterpret_cast<uint64_t *>(e->set_tab.as<char>() + 16);
         a.sets.cap = e->sets_cap;
@@ -1308,7 +1309,7 @@ int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t ite
         a.sets.pool_cap = e->set_pool.bytes / 4;
         a.sets.items = e->set_items.as<int2>();
         a.sets.fresh = a.sets.items + ni;
-        a.sets.few = e->ci_blocks;
+        a.sets.few = 6 * e->num_sms;
     }
     if (e->strata_level && d >= 1) {
         RET(e->strata_refs.ensure((size_t)std::max<int64_t>(items, 1) * sizeof(int4)));
@@ -1422,7 +1423,7 @@ int run_waves_graph(fpgm_engine *e, double alpha, int d, int64_t n_active, fpgm_
         if (a.strata_card) per_wave += launch_strata(e, a);
         if (a.slot_mem) per_wave += launch_compact(e, a, e->n_slots);
         wave_stamp_kernel<<<1, 1, 0, e->stream>>>(ctl, 1);
-        wave_reduce_kernel<<<blocks_for(n_active, 256), 256, 0, e->stream>>>(
+        wave_reduce_kernel<<<reduce_blocks(n_active, e->num_sms), 256, 0, e->stream>>>(
             (int)n_active, e->off.as<int32_t>(), e->flag.as<uint8_t>(), e->status.as<uint8_t>(),
             e->next.as<uint64_t>(), e->total.as<uint64_t>(), e->seprank.as<uint64_t>(), dstat);
         wave_tail_kernel<<<1, 1, 0, e->stream>>>(ctl, dstat, h);
@@ -1563,7 +1564,7 @@ int run_waves_and_count(fpgm_engine *e, double alpha, int d, int64_t n_active, f
         }
         CK(cudaEventRecord(e->ev2, e->stream));
         CK(cudaMemsetAsync(dstat + ST_UNRESOLVED, 0, 8, e->stream));
-        wave_reduce_kernel<<<blocks_for(n_active, 256), 256, 0, e->stream>>>(
+        wave_reduce_kernel<<<reduce_blocks(n_active, e->num_sms), 256, 0, e->stream>>>(
             (int)n_active, e->off.as<int32_t>(), e->flag.as<uint8_t>(), e->status.as<uint8_t>(),
             e->next.as<uint64_t>(), e->total.as<uint64_t>(), e->seprank.as<uint64_t>(), dstat);
         CK(cudaGetLastError());

@@ -7,7 +7,7 @@
 // is scored from its set's table with the strides of its own x, y and Z.
 //   classify        enters the test's set (set_enter); a set met for the first time gets room
 //                   for its table and goes to the list of sets to count
-//   set_count_*     one warp (tables of at most WaveArgs::warp_ints) or one CTA per new set
+//   set_count_*     one to eight warps per new set
 //   set_score_*     one warp or one CTA per test
 // Tests per distinct set, duplicates of a pair included: 1.2 (1,041 variables, level 1), 1.6 to
 // 2.0 (100 to 223 variables, level 1), 2 to 2.3 at level 2, 3.3 to 3.8 at level 3, 4.8 at level 4.
@@ -15,13 +15,6 @@
 #include "ci_kernels.cuh"
 
 namespace fpgm {
-
-// Replicas (log2) of a counted table interleaved cell by cell, as many as fit `ints`.
-__device__ __forceinline__ int replica_log(int cells, int extra, int ints) {
-    for (int l = 5; l >= 1; --l)
-        if ((cells << l) + extra <= ints) return l;
-    return 0;
-}
 
 // Warp or CTA: the variables of an item in ascending order (rank of each of z.., x, y among
 // them), their columns and state counts, and the stride of each in the set's table.
@@ -51,87 +44,119 @@ __device__ inline void set_shape(const WaveArgs &a, int item, int lane, SetShape
     __syncwarp();
 }
 
-// One warp per new set.  Bound by instruction issue (4.5 per sample and set of three columns)
-// and the shared-memory atomic unit; the samples come from L2.
-template <int kSlice, int kMinBlocks>
-__global__ void __launch_bounds__(kThreads, kMinBlocks) set_count_warp_kernel(WaveArgs a) {
-    extern __shared__ int smem[];
-    __shared__ SetShape s_shape[kWarps];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int *rep = smem + warp * kSlice;
-    SetShape &sh = s_shape[warp];
-    const int n0 = a.counters[C_SETW], ncols = a.d + 2;
-    if (n0 <= a.sets.few) return;  // set_count_cta_kernel takes them
-    for (;;) {
-        int idx = 0;
-        if (lane == 0) idx = atomicAdd(&a.counters[C_WSETW], 1);
-        idx = __shfl_sync(0xffffffffu, idx, 0);
-        if (idx >= n0) break;
-        const int2 e = a.sets.fresh[idx];  // set, an item of it
-        const int64_t S = a.var_S[a.item_vars[(int64_t)e.y * ncols]];
-        set_shape(a, e.y, lane, sh);
-        const int cells = sh.stride[0] * (int)sh.dim[0];
-        const int lgR = replica_log(cells, 0, kSlice);
-        for (int i = lane; i < (cells << lgR); i += 32) rep[i] = 0;
-        __syncwarp();
-        // lane l counts into replica l mod R: with 32 replicas every lane owns one bank
-        count_columns<32>(rep, lgR, lane, sh.col, sh.dim, ncols, S, lane);
-        __syncwarp();
-        int *out = a.sets.pool + a.sets.off[e.x];
-        long long h = 0;
-        for (int c = lane; c < cells; c += 32) {
-            int n = 0;
-            for (int r = 0; r < (1 << lgR); ++r) n += rep[(c << lgR) + ((r + lane) & ((1 << lgR) - 1))];
-            out[c] = n;
-            h += __ldg(&a.fx.f[n]);
-        }
-        h = warp_sum_ll(h);
-        if (lane == 0) a.sets.h[e.x] = h;
-        __syncwarp();
-    }
+template <int kWarpsPer>
+__device__ __forceinline__ void warps_sync(int group) {
+    if (kWarpsPer == 1) __syncwarp();
+    else if (kWarpsPer == kWarps) __syncthreads();
+    else asm volatile("bar.sync %0, %1;" ::"r"((kWarpsPer == 4 ? 1 : 3) + group), "n"(32 * kWarpsPer) : "memory");
 }
 
-// One CTA per new set whose table is beyond a warp's slice, and for every new set of a wave with
-// no more of them than CTAs: a warp would count 500,000 samples in about 100 us while the rest
-// of the GPU waits.
-__global__ void __launch_bounds__(kThreads, 2) set_count_cta_kernel(WaveArgs a) {
+// Counts the set of entry e.x (shape of item e.y in sh) with n threads, and writes its table in
+// the order of its ascending variables; returns the thread's share of the sum of F.
+template <class Sync>
+__device__ __forceinline__ long long count_set(const WaveArgs &a, const int2 e, const SetShape &sh, int64_t S, int *rep,
+                                               int ints, int t, int n, const Sync &sync) {
+    const int cells = sh.stride[0] * (int)sh.dim[0], lane = threadIdx.x & 31;
+    const int lgR = set_replicas(cells, S, ints), R = 1 << lgR;
+    for (int i = t; i < (cells << lgR); i += n) rep[i] = 0;
+    sync();
+    count_columns(rep, lgR, lane, sh.col, sh.dim, a.d + 2, S, t, n);
+    sync();
+    int *out = a.sets.pool + a.sets.off[e.x];
+    long long h = 0;
+    for (int c = t; c < cells; c += n) {
+        int m = 0;
+        for (int r = 0; r < R; ++r) m += rep[(c << lgR) + ((r + lane) & (R - 1))];
+        out[c] = m;
+        h += __ldg(&a.fx.f[m]);
+    }
+    return h;
+}
+
+// The sets of one class, kWarpsPer warps each.
+template <int kWarpsPer>
+__device__ inline void count_sets(const WaveArgs &a, int *smem, SetShape *s_shape, int2 *s_e, long long *s_h, int k) {
+    const int group = (threadIdx.x >> 5) / kWarpsPer, t = threadIdx.x % (32 * kWarpsPer), lane = threadIdx.x & 31;
+    const int first = group * kWarpsPer;  // the group's first warp: its shared memory is theirs
+    int *rep = smem + first * kSetWarpInts;
+    SetShape &sh = s_shape[first];
+    const int n = a.counters[C_SET + k];
+    auto sync = [&]() { warps_sync<kWarpsPer>(group); };
+    for (;;) {
+        if (t < 32) {
+            int idx = 0;
+            if (lane == 0) idx = atomicAdd(&a.counters[C_WSET + k], 1);
+            idx = __shfl_sync(0xffffffffu, idx, 0);
+            const int2 e = idx < n ? a.sets.fresh[k * a.list_cap + idx] : make_int2(-1, 0);
+            if (e.x >= 0) set_shape(a, e.y, lane, sh);
+            if (lane == 0) {
+                s_e[first] = e;
+                s_h[first] = 0;
+            }
+        }
+        sync();
+        const int2 e = s_e[first];
+        if (e.x < 0) break;
+        const int64_t S = a.var_S[a.item_vars[(int64_t)e.y * (a.d + 2)]];
+        const long long h = warp_sum_ll(count_set(a, e, sh, S, rep, kSetWarpInts * kWarpsPer, t, 32 * kWarpsPer, sync));
+        if (kWarpsPer == 1) {
+            if (lane == 0) a.sets.h[e.x] = h;
+        } else if (lane == 0) {
+            atomicAdd(reinterpret_cast<unsigned long long *>(&s_h[first]), (unsigned long long)h);
+        }
+        sync();
+        if (kWarpsPer > 1) {
+            if (t == 0) a.sets.h[e.x] = s_h[first];
+        }
+    }
+    sync();  // s_e and the group's shared memory are free
+}
+
+// New sets of tables of up to 8 * kSetWarpInts cells, 8, 4, 2 or 1 warps each (set_class); in a
+// wave of few sets the whole CTA counts each, so that no warp is left alone with all samples of
+// one.  Bound by the shared-memory atomics and instruction issue together; the samples come
+// from L2.
+__global__ void __launch_bounds__(kThreads, 3) set_count_kernel(WaveArgs a) {
+    extern __shared__ int smem[];
+    __shared__ SetShape s_shape[kWarps];
+    __shared__ int2 s_e[kWarps];
+    __shared__ long long s_h[kWarps];
+    const int small = a.counters[C_SET] + a.counters[C_SET + 1] + a.counters[C_SET + 2];
+    count_sets<8>(a, smem, s_shape, s_e, s_h, 3);
+    if (small <= a.sets.few) {
+        for (int k = 2; k >= 0; --k) count_sets<8>(a, smem, s_shape, s_e, s_h, k);
+        return;
+    }
+    count_sets<4>(a, smem, s_shape, s_e, s_h, 2);
+    count_sets<2>(a, smem, s_shape, s_e, s_h, 1);
+    count_sets<1>(a, smem, s_shape, s_e, s_h, 0);
+}
+
+// One CTA per new set of a larger table.
+__global__ void __launch_bounds__(kThreads, 2) set_count_big_kernel(WaveArgs a) {
     extern __shared__ int smem[];
     __shared__ SetShape sh;
     __shared__ int s_idx;
-    __shared__ long long s_h;
+    __shared__ unsigned long long s_h;
     const int tid = threadIdx.x, lane = tid & 31;
-    const int n1 = a.counters[C_SETC], ncols = a.d + 2;
-    const int n0 = a.counters[C_SETW] <= a.sets.few ? a.counters[C_SETW] : 0;
+    const int n = a.counters[C_SET + 4];
     for (;;) {
         if (tid == 0) {
-            s_idx = atomicAdd(&a.counters[C_WSETC], 1);
+            s_idx = atomicAdd(&a.counters[C_WSET + 4], 1);
             s_h = 0;
         }
         __syncthreads();
         const int idx = s_idx;
-        if (idx >= n1 + n0) break;
-        const int2 e = a.sets.fresh[idx < n1 ? a.list_cap - 1 - idx : idx - n1];
-        const int64_t S = a.var_S[a.item_vars[(int64_t)e.y * ncols]];
+        if (idx >= n) break;
+        const int2 e = a.sets.fresh[4 * a.list_cap + idx];
+        const int64_t S = a.var_S[a.item_vars[(int64_t)e.y * (a.d + 2)]];
         if (tid < 32) set_shape(a, e.y, lane, sh);
         __syncthreads();
-        const int cells = sh.stride[0] * (int)sh.dim[0];
-        const int lgR = replica_log(cells, 0, kCtaInts);
-        for (int i = tid; i < (cells << lgR); i += kThreads) smem[i] = 0;
+        const long long h =
+            warp_sum_ll(count_set(a, e, sh, S, smem, kCtaInts, tid, kThreads, []() { __syncthreads(); }));
+        if (lane == 0) atomicAdd(&s_h, (unsigned long long)h);
         __syncthreads();
-        count_columns<kThreads>(smem, lgR, lane, sh.col, sh.dim, ncols, S, tid);
-        __syncthreads();
-        int *out = a.sets.pool + a.sets.off[e.x];
-        long long h = 0;
-        for (int c = tid; c < cells; c += kThreads) {
-            int n = 0;
-            for (int r = 0; r < (1 << lgR); ++r) n += smem[(c << lgR) + ((r + lane) & ((1 << lgR) - 1))];
-            out[c] = n;
-            h += __ldg(&a.fx.f[n]);
-        }
-        h = warp_sum_ll(h);
-        if (lane == 0) atomicAdd(reinterpret_cast<unsigned long long *>(&s_h), (unsigned long long)h);
-        __syncthreads();
-        if (tid == 0) a.sets.h[e.x] = s_h;
+        if (tid == 0) a.sets.h[e.x] = (long long)s_h;
         __syncthreads();
     }
 }
