@@ -752,7 +752,7 @@ extern "C" int fpgm_engine_create(int32_t device, fpgm_engine **out) {
                             kWarps * kWarpIntsSmall * 4));
     CK(cudaFuncSetAttribute(set_count_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     CK(cudaFuncSetAttribute(set_score_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    CK(cudaFuncSetAttribute(strata_test_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStrataInts * 4));
+    CK(cudaFuncSetAttribute(strata_test_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTestInts * 4));
     CK(cudaFuncSetAttribute(ci_plain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     int occ = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ci_warp_kernel<kWarpInts, 2>, kThreads, kSmemBytes));
@@ -1132,7 +1132,7 @@ int launch_shared_tiers(fpgm_engine *e, const WaveArgs &a) {
 // ---- shared strata (strata.cuh)
 // Tables: keys of nodes and pairs, then their fields; all sized by the two capacities.
 constexpr int kStrataNodes = 1 << 19, kStrataPairs = 1 << 20, kStrataBuild = 1 << 17;
-constexpr size_t kStrataKeyBytes = (size_t)kStrataNodes * 8 + (size_t)kStrataPairs * 8;
+constexpr size_t kStrataKeyBytes = (size_t)kStrataNodes * 8 + (size_t)kStrataPairs * 12;  // and the pairs' lists
 
 void strata_args(fpgm_engine *e, StrataArgs &s) {
     memset(&s, 0, sizeof s);
@@ -1144,6 +1144,7 @@ void strata_args(fpgm_engine *e, StrataArgs &s) {
     };
     s.node_key = reinterpret_cast<uint64_t *>(take((size_t)kStrataNodes * 8));
     s.pair_key = reinterpret_cast<uint64_t *>(take((size_t)kStrataPairs * 8));
+    s.pair_head = reinterpret_cast<int32_t *>(take((size_t)kStrataPairs * 4));
     s.node_h = reinterpret_cast<long long *>(take((size_t)kStrataNodes * 8));
     s.node_ids = reinterpret_cast<int64_t *>(take((size_t)kStrataNodes * 8));
     s.pair_h = reinterpret_cast<long long *>(take((size_t)kStrataPairs * 8));
@@ -1160,7 +1161,11 @@ void strata_args(fpgm_engine *e, StrataArgs &s) {
     s.build_cap = kStrataBuild;
     s.pair_list = s.build_list + (size_t)(kStrataMaxSets + 1) * kStrataBuild;
     s.pair_list_cap = kStrataPairs;
+    const size_t items = e->strata_refs.bytes / (2 * sizeof(int4) + 8);
     s.item_ref = e->strata_refs.as<int4>();
+    s.pack_list = s.item_ref + items;
+    s.item_next = reinterpret_cast<int32_t *>(s.pack_list + items);
+    s.group_list = s.item_next + items;
 }
 
 // Level d's waves count through shared strata when a test can go past shared memory: buffers
@@ -1221,8 +1226,10 @@ int launch_strata(fpgm_engine *e, const WaveArgs &a) {
     for (int size = 1; size <= a.d + 1; ++size)
         strata_count_kernel<true><<<grid, kStrataThreads, kStrataInts * 4, e->stream>>>(a, s, size);
     strata_count_kernel<false><<<grid, kStrataThreads, kStrataInts * 4, e->stream>>>(a, s, 0);
-    strata_test_kernel<<<grid, kStrataThreads, kStrataInts * 4, e->stream>>>(a, s);
-    return a.d + 4;
+    const int ctas = 5 * e->num_sms;
+    strata_pack_kernel<<<e->num_sms, 128, 0, e->stream>>>(a, s, ctas);
+    strata_test_kernel<<<ctas, kTestThreads, kTestInts * 4, e->stream>>>(a, s);
+    return a.d + 5;
 }
 
 int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t items) {
@@ -1312,7 +1319,7 @@ int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t ite
         a.sets.few = 6 * e->num_sms;
     }
     if (e->strata_level && d >= 1) {
-        RET(e->strata_refs.ensure((size_t)std::max<int64_t>(items, 1) * sizeof(int4)));
+        RET(e->strata_refs.ensure((size_t)std::max<int64_t>(items, 1) * (2 * sizeof(int4) + 8)));
         a.strata_card = kStrataMaxCard;
     }
     a.part_max_log = e->part_max_log;
