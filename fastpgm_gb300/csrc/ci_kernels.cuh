@@ -170,6 +170,10 @@ struct WaveArgs {
     unsigned long long *stats;
     double alpha;
     BandTables bt;
+    const uint32_t *bits;  // the level's adjacency, bit_words words per variable
+    int32_t bit_words;
+    float *pair_g2;        // level 0's statistics, n_vars x n_vars (null: not kept); level 1 reads them
+    int32_t n_vars;
     Fixed fx;              // fixed-point statistic of tests that need no detail
     SetArgs sets;
     int32_t strata_card;   // tests whose other endpoint has at most this many states go to list 6 (0: none)
@@ -337,15 +341,43 @@ __host__ __device__ inline int set_class(int cells, int64_t S) {
     return k;
 }
 
-// Entry of the set of m >= 3 ascending variables: the first three in one key, then two at a
+// Entry of the set of m >= 2 ascending variables: the first three in one key, then two at a
 // time after the entry reached so far (the keys hold the variables themselves, so two sets
 // never share an entry).  -1: no room.
 __device__ inline int set_enter(const SetArgs &s, const uint16_t *v, int m, bool *fresh) {
-    int at = table_enter(s.key, s.cap, s.probe, (1ull << 62) | (uint64_t)v[0] << 32 | (uint64_t)v[1] << 16 | v[2], fresh);
+    int at = table_enter(s.key, s.cap, s.probe, (1ull << 62) | (uint64_t)v[0] << 32 | (uint64_t)v[1] << 16 | (m > 2 ? v[2] : 0xffffu),
+                         fresh);
     for (int i = 3; i < m && at >= 0; i += 2)
         at = table_enter(s.key, s.cap, s.probe,
                          (1ull << 63) | (uint64_t)at << 32 | (uint64_t)v[i] << 16 | (i + 1 < m ? v[i + 1] : 0xffffu), fresh);
     return at;
+}
+
+// Tests whose outcome needs no count.
+// A test from y's side whose Z lies inside x's neighbours too was a test from x's side: had it
+// been independent, the edge's first independent rank would be that one.
+__device__ inline bool tested_from_x(const WaveArgs &a, int x, const int *z) {
+    const uint32_t *row = a.bits + (int64_t)x * a.bit_words;
+    bool in = true;
+    for (int k = 0; k < a.d; ++k) in = in && ((__ldg(row + (z[k] >> 5)) >> (z[k] & 31)) & 1u);
+    return in;
+}
+// Dependent by the chain rule of mutual information.  I(x; y | z) = I(x; y) + I(x; z | y) - I(x; z) is
+// at least I(x; y) - min(I(x; z), I(y; z)), and G^2 is 2 S times the information of the observed
+// frequencies, so level 0's statistics bound level 1's from below.  Past the quantile of the
+// largest degrees of freedom the test can have, it is dependent.  The floats' rounding is in the
+// margin.  Of the tests of level 1 this decides 57% (100 variables x 50,000 samples), 69% (223 x
+// 500,000) and 68% (1,041 x 100,000); tested_from_x 26%, 17% and 8%.
+__device__ inline bool dependent_by_pairs(const WaveArgs &a, int x, int y, int z, int64_t df) {
+    if (df > a.fx.dfmax) return false;
+    const float *gx = a.pair_g2 + (int64_t)x * a.n_vars, *gy = a.pair_g2 + (int64_t)y * a.n_vars;
+    const double xy = gx[y], xz = gx[z], yz = gy[z];
+    const double low = xy - fmin(xz, yz);
+    return low - 1e-6 * (xy + xz + yz) - 1e-3 > a.fx.hi[df];
+}
+__device__ inline void keep_pair(const WaveArgs &a, int x, int y, double g2) {
+    a.pair_g2[(int64_t)x * a.n_vars + y] = (float)g2;
+    a.pair_g2[(int64_t)y * a.n_vars + x] = (float)g2;
 }
 
 // Item -> (x, y, Z) -> tier.  One thread per item, grid-stride.
@@ -383,6 +415,16 @@ __global__ void classify_kernel(WaveArgs a) {
                 for (int k = 0; k < d; ++k) z[k] = L[c[k] < skip ? c[k] : c[k] + 1];
             }
         }
+        if (kSource == SRC_WAVE && d > 0) {
+            const bool known =
+                (side == 1 && a.bits && tested_from_x(a, x, z)) ||
+                (d == 1 && a.pair_g2 &&
+                 dependent_by_pairs(a, x, y, z[0], (int64_t)(a.card[x] - 1) * (a.card[y] - 1) * a.card[z[0]]));
+            if (known) {
+                a.flag[item] = 0;
+                continue;
+            }
+        }
         uint16_t *iv = a.item_vars + (int64_t)item * ncols;
         double dzf = 1.0;
         int64_t dz = 1;
@@ -409,7 +451,7 @@ __global__ void classify_kernel(WaveArgs a) {
             continue;
         }
         bool placed = false;
-        if (kSource == SRC_WAVE && tier < 2 && a.sets.key != nullptr && d > 0) {
+        if (kSource == SRC_WAVE && tier < 2 && a.sets.key != nullptr) {
             uint16_t sv[kMaxCols];  // the set, ascending (x < y, z ascending)
             for (int k = 0, i = 0, j = 0; k < ncols; ++k) {
                 const int p = j == 0 ? x : y;

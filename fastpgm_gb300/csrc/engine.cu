@@ -139,6 +139,7 @@ struct DevBuf {
     }
 };
 
+constexpr int kPairVars = 8192;                        // level 0's statistics are kept up to here (256 MB)
 constexpr int kStatusActive = 0, kStatusRemoved = 1, kStatusKept = 2;
 constexpr int64_t kPlainInts = (int64_t)1 << 25;       // plain kernel's global table (128 MB)
 constexpr int64_t kMaxItems = (int64_t)1 << 22;        // tests per wave
@@ -227,6 +228,8 @@ struct fpgm_engine {
     unsigned long long sets_used = 0;   // ints of tables the last level asked for
     size_t set_pool_fixed = 0, strata_pool_fixed = 0;  // FPGM_SET_POOL, FPGM_STRATA_POOL (tests): bytes
     DevBuf set_tab, set_pool, set_items;
+    DevBuf pair_g2;                     // level 0's statistics, read at level 1 (FPGM_BOUND=0: not kept)
+    bool bound_on = true, pairs_kept = false;
     bool tune_loaded = false, tune_online = true;
     std::string tune_source;
     // result
@@ -669,7 +672,10 @@ __global__ void __launch_bounds__(kThreads) level0_gram_score_kernel(WaveArgs a,
         const Verdict v = a.fx.f ? score_fixed(g, tab, nullptr, dy, 1, dx, dy, 1, ni, nj, nk, nullptr, a.fx, a.alpha,
                                                a.var_S[x], nullptr)
                                  : score_dense(g, tab, ni, nj, nk, dx, dy, 1, a.alpha, a.bt, false, false, nullptr);
-        if (lane == 0) record(a, item, v, cells, 0, 0);
+        if (lane == 0) {
+            record(a, item, v, cells, 0, 0);
+            if (a.fx.f && a.pair_g2) keep_pair(a, x, y, v.g2);
+        }
         __syncwarp();
     }
 }
@@ -785,6 +791,7 @@ extern "C" int fpgm_engine_create(int32_t device, fpgm_engine **out) {
     if (const char *w = getenv("FPGM_GRAPH")) e->graph_on = atoi(w) != 0;
     if (const char *w = getenv("FPGM_STRATA")) e->strata_on = atoi(w) != 0;
     if (const char *w = getenv("FPGM_SETS")) e->sets_on = atoi(w) != 0;
+    if (const char *w = getenv("FPGM_BOUND")) e->bound_on = atoi(w) != 0;
     if (const char *w = getenv("FPGM_SET_POOL")) e->set_pool_fixed = (size_t)std::max(16ll, atoll(w));
     if (const char *w = getenv("FPGM_STRATA_POOL")) e->strata_pool_fixed = (size_t)std::max(16ll, atoll(w));
     e->gram = gram_create();
@@ -832,7 +839,7 @@ extern "C" int fpgm_engine_destroy(fpgm_engine *e) {
                       &e->tune_obs, &e->ovf, &e->live_pool[0], &e->live_pool[1], &e->live_tab[0], &e->live_tab[1],
                       &e->live_cnt, &e->live_stat, &e->res_adj_d, &e->res_key, &e->res_idx, &e->res_removed_d, &e->res_cnt,
                       &e->res_vars_d, &e->fixed_f, &e->tight, &e->set_tab,
-                      &e->set_pool, &e->set_items, &e->strata_tab, &e->strata_lists, &e->strata_pool,
+                      &e->set_pool, &e->set_items, &e->pair_g2, &e->strata_tab, &e->strata_lists, &e->strata_pool,
                       &e->strata_refs, &e->strata_used};
     for (DevBuf *b : bufs) b->release();
     gram_destroy(e->gram);
@@ -1080,7 +1087,7 @@ int fixed_setup(fpgm_engine *e) {
 constexpr size_t kSetPoolMax = (size_t)4 << 30;
 int sets_setup(fpgm_engine *e, int d, int64_t n_active) {
     e->sets_level = false;
-    if (!e->sets_on || e->fixed_n < e->S || d < 1 || e->wave_log || e->phase_timers.p) return FPGM_OK;
+    if (!e->sets_on || e->fixed_n < e->S || e->wave_log || e->phase_timers.p) return FPGM_OK;
     const int64_t tests = std::min<int64_t>(e->level_tests, 64 * n_active);
     int32_t cap = 1 << 12;
     while (cap < 4 * tests && cap < (1 << 22)) cap <<= 1;
@@ -1246,7 +1253,7 @@ int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t ite
     const int64_t df = max_table_ints(e->h_card, d);  // a test's degrees of freedom are below its table's size
     // the FP32 statistic's tables, unless every test of the wave is decided in fixed point
     const bool gram = d == 0 && e->n_jobs == 1 && e->gram_on && e->gram_planned && e->gram_ok;
-    if (!(e->in_skeleton && e->fixed_n >= e->S && (gram || (d >= 1 && e->sets_level && e->sets_all)))) {
+    if (!(e->in_skeleton && e->fixed_n >= e->S && (gram || (e->sets_level && e->sets_all)))) {
         RET(ensure_band(e, alpha, df));
         a.bt.lo = e->band.as<double>();
         a.bt.hi = a.bt.lo + e->band_df + 1;
@@ -1303,7 +1310,13 @@ int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t ite
             }
         }
     }
-    if (e->sets_level && d >= 1) {
+    if (e->in_skeleton) {
+        a.bits = e->bits.as<uint32_t>();
+        a.bit_words = (e->n + 31) / 32;
+        a.n_vars = e->n;
+        if (a.fx.f && d <= 1 && e->pairs_kept) a.pair_g2 = e->pair_g2.as<float>();
+    }
+    if (e->sets_level) {
         const size_t ni = (size_t)std::max<int64_t>(items, 1);
         RET(e->set_items.ensure(ni * 6 * sizeof(int2)));
         a.sets.used = e->set_tab.as<unsigned long long>();
@@ -1752,13 +1765,20 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
                 }
                 gram = e->gram_ok;
             }
+            if (d == 0) {  // every pair's statistic is kept when level 0 computes it in fixed point
+                e->pairs_kept = e->bound_on && e->fixed_n >= e->S && n <= kPairVars && !e->wave_log &&
+                                !e->phase_timers.p && (gram || (e->sets_on && e->n_jobs > 1)) &&
+                                max_table_ints(e->h_card, 0) * 2 <= kCtaInts &&
+                                e->pair_g2.ensure((size_t)n * n * sizeof(float)) == FPGM_OK;
+            }
             if (!gram) RET(live_setup(e, d));
             {  // a test per rank: at most C(max_deg - 1, d) from either side of an edge
                 double c = 2.0 * (double)n_active;
                 for (int k = 0; k < d; ++k) c = std::min(1e15, c * std::max(0, max_deg - 1 - k) / (k + 1));
                 e->level_tests = d == 0 ? n_active : (int64_t)c + 64;
             }
-            RET(sets_setup(e, d, n_active));
+            if (!gram) RET(sets_setup(e, d, n_active));
+            if (d == 0 && !gram && !(e->sets_level && e->sets_all)) e->pairs_kept = false;  // some tests count their own
             RET(strata_setup(e, d, d <= 1));
             RET(run_waves_and_count(e, alpha, d, n_active, st, st->n_levels, a, gram));
             if (e->live_on && e->live_stat.p) {

@@ -216,7 +216,10 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) set_score_warp_kernel(Wa
         __syncwarp();
         const Verdict v = score_fixed(g, tab, zoff, sh.stride[rx], sh.stride[ry], dx, dy, dz, ni, nj, nk,
                                       a.sets.h + e.x, a.fx, a.alpha, S, nullptr);
-        if (lane == 0) record(a, e.y, v, cells, 0, 0);
+        if (lane == 0) {
+            record(a, e.y, v, cells, 0, 0);
+            if (d == 0 && a.pair_g2) keep_pair(a, a.item_vars[(int64_t)e.y * 2], a.item_vars[(int64_t)e.y * 2 + 1], v.g2);
+        }
         __syncwarp();
     }
 }
@@ -252,7 +255,10 @@ __global__ void __launch_bounds__(kThreads, 2) set_score_cta_kernel(WaveArgs a) 
         __syncthreads();
         const Verdict v = score_fixed(g, smem, zoff, sh.stride[rx], sh.stride[ry], dx, dy, dz, ni, nj, nk,
                                       a.sets.h + e.x, a.fx, a.alpha, S, scratch);
-        if (tid == 0) record(a, e.y, v, cells, 0, 1);
+        if (tid == 0) {
+            record(a, e.y, v, cells, 0, 1);
+            if (d == 0 && a.pair_g2) keep_pair(a, a.item_vars[(int64_t)e.y * 2], a.item_vars[(int64_t)e.y * 2 + 1], v.g2);
+        }
         __syncthreads();
     }
 }

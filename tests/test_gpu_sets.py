@@ -60,3 +60,33 @@ def test_constant_and_equal_columns():
     raw[5] = raw[4]
     raw[7] = (raw[1] + raw[6]) % 3
     _check(raw)
+
+
+@pytest.mark.parametrize("bound", ["1", "0"])
+@pytest.mark.parametrize("n,S,card,edges,alpha", [(40, 3000, (2, 3), 70, 0.05), (30, 20000, (2, 9), 45, 0.05),
+                                                  (25, 4000, (2, 4), 60, 0.0), (25, 4000, (2, 4), 60, 0.9),
+                                                  (20, 500, (2, 2), 40, 1e-4)])
+def test_level_1_bounds_match_oracle(monkeypatch, bound, n, S, card, edges, alpha):
+    """Level 1 decided from level 0's statistics where the chain rule allows (FPGM_BOUND=0: every
+    test counted): near-copies of a variable put the bound close to the threshold."""
+    monkeypatch.setenv("FPGM_BOUND", bound)
+    raw, _, _ = F.generate(n_nodes=n, n_samples=S, seed=n + S, n_edges=edges, max_indegree=4, card=card)
+    rng = np.random.default_rng(n)
+    for v in range(0, n - 1, 5):  # noisy copies: strongly dependent pairs through a common neighbour
+        keep = rng.random(S) < rng.uniform(0.05, 0.9)
+        raw[v + 1, keep] = raw[v, keep]
+    _check(raw, depth=4, alpha=alpha)
+
+
+def test_level_1_bounds_across_datasets():
+    data = [F.generate(n_nodes=n, n_samples=S, seed=S, n_edges=2 * n, max_indegree=4, card=(2, 5))[0]
+            for n, S in ((12, 700), (30, 9000), (2, 40), (17, 2500))]
+    with F.Engine(0) as e:
+        e.upload_jobs(data)
+        e.pc_skeleton()
+        res = e.result()
+        offsets = e.job_offsets
+    for raw, (adj, seps) in zip(data, F.split_jobs(res, offsets)):
+        cols, card = O.relabel(raw)
+        ref = O.pc_skeleton(cols, card, threads=16)
+        assert np.array_equal(adj, ref["adj"]) and seps == ref["sepsets"]
