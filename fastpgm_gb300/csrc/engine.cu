@@ -146,8 +146,13 @@ constexpr int64_t kMaxItems = (int64_t)1 << 22;        // tests per wave
 
 }  // namespace
 
+namespace {
+struct LevelHost;
+}
+
 struct fpgm_engine {
     int device = 0;
+    LevelHost *level_host = nullptr;  // pinned: what a level leaves for the host
     cudaStream_t stream = nullptr;
     int num_sms = 0, ci_blocks = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
@@ -433,17 +438,39 @@ __global__ void wave_plan_kernel(int n_edges, const uint8_t *status, const uint6
     g[e] = v;
 }
 
-// One warp per edge: its ranks' results 32 at a time (an edge can have 4,096 in a wave).
+// Control block of the device-driven waves.
+struct WaveCtl {
+    long long wave, q, n_waves;
+    unsigned long long t_prev, count_ns, large_ns;
+    unsigned ticket;
+};
+constexpr long long kMaxWaves = 1 << 20;  // bound on waves per level (each wave resolves >= 1 rank per edge)
+
+__device__ inline unsigned long long device_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// One warp per edge: its ranks' results 32 at a time (an edge can have 4,096 in a wave).  off
+// null: one rank per edge, at its own place (level 0).  With a control block the last CTA ends the
+// wave: device times, wave count and, in a graph, whether another wave runs.  tier2: the time
+// since the last stamp is the tier-2 kernels', else the shared-memory tiers'.
 __global__ void wave_reduce_kernel(int n_edges, const int32_t *off, const uint8_t *flag, uint8_t *status,
                                    uint64_t *next, const uint64_t *total, uint64_t *seprank,
-                                   unsigned long long *stats) {
+                                   unsigned long long *stats, WaveCtl *ctl, int tier2, int in_graph,
+                                   cudaGraphConditionalHandle h) {
     __shared__ unsigned long long s_sum[4];  // bad, executed, deterministic, unresolved
     const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
     if (threadIdx.x < 4) s_sum[threadIdx.x] = 0;
+    if (ctl && blockIdx.x == 0 && threadIdx.x == 0) {
+        const unsigned long long t = device_ns();
+        (tier2 ? ctl->large_ns : ctl->count_ns) += t - ctl->t_prev;
+    }
     __syncthreads();
     unsigned long long bad = 0, exec = 0, det = 0, unresolved = 0;  // lane 0's
     for (int e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < n_edges; e += warps) {
-        const int o = off[e], g = off[e + 1] - o;
+        const int o = off ? off[e] : e, g = off ? off[e + 1] - o : 1;
         if (g <= 0) continue;
         int first = -1;
         for (int k0 = 0; k0 < g && first < 0; k0 += 32) {
@@ -480,20 +507,29 @@ __global__ void wave_reduce_kernel(int n_edges, const int32_t *off, const uint8_
                          : threadIdx.x == 2 ? ST_DET
                                             : ST_UNRESOLVED],
                   s_sum[threadIdx.x]);
+    if (!ctl) return;
+    __threadfence();  // the block's sums are visible before it counts as done
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&ctl->ticket, 1u) == gridDim.x - 1) {
+        __threadfence();
+        ctl->ticket = 0;
+        ctl->wave += 1;
+        ctl->n_waves += 1;
+        const bool more = *(volatile unsigned long long *)&stats[ST_UNRESOLVED] > 0 &&
+                          *(volatile unsigned long long *)&stats[ST_UNSUPPORTED] == 0 && ctl->wave < kMaxWaves;
+        if (in_graph) cudaGraphSetConditional(h, more ? 1u : 0u);
+    }
 }
 inline int reduce_blocks(int64_t n_edges, int num_sms) {
     return (int)std::min<int64_t>((n_edges + 7) / 8, 8 * (int64_t)num_sms);
 }
 
 // apply removals, log (pair, sepset) -- sepset rebuilt from its rank
-__global__ void level_finalize_kernel(int n_edges, int d, int W, const int32_t *ex, const int32_t *ey,
-                                      const int32_t *pxy, const int32_t *pyx, const uint64_t *cntx,
-                                      const uint64_t *seprank, const uint8_t *status, const int32_t *adjl,
-                                      int stride, const int32_t *deg, const uint64_t *btab, uint32_t *bits,
-                                      int32_t *log_pair, int32_t *log_meta, int32_t *log_vars, int64_t log_base,
-                                      int64_t var_base, unsigned long long *stats) {
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_edges) return;
+__device__ inline void finalize_edge(int e, int d, int W, const int32_t *ex, const int32_t *ey, const int32_t *pxy,
+                                     const int32_t *pyx, const uint64_t *cntx, const uint64_t *seprank,
+                                     const uint8_t *status, const int32_t *adjl, int stride, const int32_t *deg,
+                                     const uint64_t *btab, uint32_t *bits, int32_t *log_pair, int32_t *log_meta,
+                                     int32_t *log_vars, int64_t log_base, int64_t var_base, unsigned long long *stats) {
     if (status[e] != kStatusRemoved) return;
     const int x = ex[e], y = ey[e];
     atomicAnd(&bits[(int64_t)x * W + (y >> 5)], ~(1u << (y & 31)));
@@ -518,6 +554,24 @@ __global__ void level_finalize_kernel(int n_edges, int d, int W, const int32_t *
     unrank_lex(btab, deg[side_node] - 1, d, rank, c);
     const int32_t *L = adjl + (int64_t)side_node * stride;
     for (int k = 0; k < d; ++k) log_vars[var_base + slot * d + k] = L[c[k] < skip ? c[k] : c[k] + 1];
+}
+
+__global__ void level_finalize_kernel(int n_edges, int d, int W, const int32_t *ex, const int32_t *ey,
+                                      const int32_t *pxy, const int32_t *pyx, const uint64_t *cntx,
+                                      const uint64_t *seprank, const uint8_t *status, const int32_t *adjl,
+                                      int stride, const int32_t *deg, const uint64_t *btab, uint32_t *bits,
+                                      int32_t *log_pair, int32_t *log_meta, int32_t *log_vars, int64_t log_base,
+                                      int64_t var_base, unsigned long long *stats, int with_degrees, int n) {
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n_edges; e += gridDim.x * blockDim.x)
+        finalize_edge(e, d, W, ex, ey, pxy, pyx, cntx, seprank, status, adjl, stride, deg, btab, bits, log_pair, log_meta,
+                      log_vars, log_base, var_base, stats);
+    if (!with_degrees) return;  // one CTA: the largest degree left, too
+    __syncthreads();
+    for (int v = threadIdx.x; v < n; v += blockDim.x) {
+        int dg = 0;
+        for (int w = 0; w < W; ++w) dg += __popc(__ldcg(bits + (int64_t)v * W + w));
+        atomicMax(&stats[ST_MAXDEG], (unsigned long long)dg);
+    }
 }
 
 __global__ void degree_kernel(const uint32_t *bits, int n, int W, unsigned long long *stats) {
@@ -570,21 +624,11 @@ __global__ void log_vars_kernel(int R, const int32_t *order, const int32_t *log_
 }
 
 // ---- device-driven wave loop (one CUDA graph per level: a WHILE conditional node whose body
-// is one wave; the wave's tail kernel decides whether another wave runs)
-struct WaveCtl {
-    long long wave, q, n_waves;
-    unsigned long long t_prev, count_ns, large_ns;
-};
-constexpr long long kMaxWaves = 1 << 20;  // bound on waves per level (each wave resolves >= 1 rank per edge)
-
+// is one wave; the wave's reduction decides whether another wave runs)
 // Start of a wave: q = ranks per unresolved edge this wave (the host loop's rule: doubling from
 // 1, raised so the wave fills the GPU, capped by the item buffers), counters cleared.
-__global__ void wave_prep_kernel(WaveCtl *c, unsigned long long *stats, int32_t *counters, StrataCounters *sc,
-                                 long long n_active, long long ci_blocks, long long max_items) {
-    counters[threadIdx.x] = 0;  // 32 threads, kCounterBytes
-    if (sc)
-        for (int i = threadIdx.x; i < (int)(sizeof(StrataCounters) / 4); i += 32) reinterpret_cast<int32_t *>(sc)[i] = 0;
-    if (threadIdx.x != 0) return;
+__device__ inline long long wave_begin(WaveCtl *c, unsigned long long *stats, long long n_active, long long ci_blocks,
+                                       long long max_items) {
     const long long unresolved = (long long)stats[ST_UNRESOLVED];
     stats[ST_UNRESOLVED] = 0;
     long long q = 1ll << (c->wave < 12 ? c->wave : 12);
@@ -595,7 +639,60 @@ __global__ void wave_prep_kernel(WaveCtl *c, unsigned long long *stats, int32_t 
     }
     const long long qmax = max_items / (n_active > 1 ? n_active : 1);
     q = q < qmax ? q : qmax;
-    c->q = q > 1 ? q : 1;
+    return c->q = q > 1 ? q : 1;
+}
+__device__ inline void clear_counters(int32_t *counters, StrataCounters *sc) {
+    if (threadIdx.x < kCounterBytes / 4) counters[threadIdx.x] = 0;
+    if (sc)
+        for (int i = threadIdx.x; i < (int)(sizeof(StrataCounters) / 4); i += blockDim.x)
+            reinterpret_cast<int32_t *>(sc)[i] = 0;
+}
+__global__ void wave_prep_kernel(WaveCtl *c, unsigned long long *stats, int32_t *counters, StrataCounters *sc,
+                                 long long n_active, long long ci_blocks, long long max_items) {
+    clear_counters(counters, sc);
+    if (threadIdx.x == 0) wave_begin(c, stats, n_active, ci_blocks, max_items);
+}
+
+__device__ __forceinline__ int wave_share(uint8_t status, uint64_t total, uint64_t next, uint64_t q) {
+    if (status != kStatusActive) return 0;
+    const uint64_t rem = total - next;
+    return (int)(rem < q ? rem : q);
+}
+
+// The whole start of a wave in one CTA: q, cleared counters, every edge's share of ranks and
+// their exclusive offsets.  Two passes over the edges; five launches of 2-4 us otherwise, which
+// win past kBeginEdges edges (50,090 edges, 15 waves: 16.5 ms in five launches, 17.8 in one).
+constexpr int kBeginEdges = 16384;
+__global__ void __launch_bounds__(1024) wave_begin_kernel(WaveCtl *c, unsigned long long *stats, int32_t *counters,
+                                                          StrataCounters *sc, int n_edges, const uint8_t *status,
+                                                          const uint64_t *total, const uint64_t *next, int32_t *off,
+                                                          long long ci_blocks, long long max_items) {
+    __shared__ int s_w[32];
+    __shared__ uint64_t s_q;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    clear_counters(counters, sc);
+    if (tid == 0) s_q = (uint64_t)wave_begin(c, stats, n_edges, ci_blocks, max_items);
+    __syncthreads();
+    const uint64_t q = s_q;
+    const int per = (n_edges + 1023) / 1024, b0 = min(n_edges, tid * per), b1 = min(n_edges, b0 + per);
+    int sum = 0;
+    for (int e = b0; e < b1; ++e) sum += wave_share(status[e], total[e], next[e], q);
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) s_w[warp] = incl;
+    __syncthreads();
+    int run = incl - sum;
+    for (int w = 0; w < warp; ++w) run += s_w[w];
+    for (int e = b0; e < b1; ++e) {
+        off[e] = run;
+        run += wave_share(status[e], total[e], next[e], q);
+    }
+    if (tid == 1023) off[n_edges] = run;
+    if (tid == 0) c->t_prev = device_ns();
 }
 
 __global__ void wave_plan_dev_kernel(int n_edges, const uint8_t *status, const uint64_t *total, const uint64_t *next,
@@ -606,37 +703,102 @@ __global__ void wave_plan_dev_kernel(int n_edges, const uint8_t *status, const u
         g[e] = 0;
         return;
     }
-    int v = 0;
-    if (status[e] == kStatusActive) {
-        const uint64_t q = (uint64_t)c->q, rem = total[e] - next[e];
-        v = (int)(rem < q ? rem : q);
-    }
-    g[e] = v;
+    g[e] = wave_share(status[e], total[e], next[e], (uint64_t)c->q);
 }
 
 // Device clock between kernels of a wave: slot -1 marks the start of the counting kernels,
 // 0 adds the shared-memory tiers' span, 1 the tier-2 kernels' span.
 __global__ void wave_stamp_kernel(WaveCtl *c, int slot) {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    const unsigned long long t = device_ns();
     if (slot == 0) c->count_ns += t - c->t_prev;
-    if (slot == 1) c->large_ns += t - c->t_prev;
     c->t_prev = t;
 }
 
-__global__ void wave_tail_kernel(WaveCtl *c, const unsigned long long *stats, cudaGraphConditionalHandle h) {
-    c->wave += 1;
-    c->n_waves += 1;
-    const bool more = stats[ST_UNRESOLVED] > 0 && stats[ST_UNSUPPORTED] == 0 && c->wave < kMaxWaves;
-    cudaGraphSetConditional(h, more ? 1u : 0u);
-}
-
-__global__ void wave_ctl_init_kernel(WaveCtl *c, unsigned long long *stats, long long n_active) {
+// A level's control block and counters.
+__device__ inline void level_init(WaveCtl *c, unsigned long long *stats, long long n_active) {
     c->wave = c->q = c->n_waves = 0;
     c->t_prev = c->count_ns = c->large_ns = 0;
+    c->ticket = 0;
     stats[ST_UNRESOLVED] = (unsigned long long)n_active;
-    stats[ST_BYTES_SHARED] = 0;
-    stats[ST_BYTES_LARGE] = 0;
+    stats[ST_BYTES_SHARED] = stats[ST_BYTES_LARGE] = 0;
+    stats[ST_DET] = stats[ST_EXEC] = stats[ST_REMOVED] = stats[ST_MAXDEG] = 0;
+}
+__global__ void level_init_kernel(WaveCtl *c, unsigned long long *stats, long long n_active) {
+    level_init(c, stats, n_active);
+}
+
+// A level's start in one CTA (up to kSnapNodes variables): neighbour lists and degrees from the
+// bitset, the edges x < y with their rank counts, the control block.  Otherwise csr_kernel, a
+// scan, level_edges_kernel and level_init_kernel (20 us at 37 variables, most of it launches).
+constexpr int kSnapNodes = 512;
+__global__ void __launch_bounds__(1024) level_snapshot_kernel(const uint32_t *bits, int n, int W, int d, int32_t *adjl,
+                                                              int stride, int32_t *deg, const uint64_t *btab,
+                                                              int32_t *ex, int32_t *ey, int32_t *pxy, int32_t *pyx,
+                                                              uint64_t *cntx, uint64_t *total, uint64_t *next,
+                                                              uint8_t *status, unsigned long long *stats, WaveCtl *ctl) {
+    __shared__ int s_higher[kSnapNodes + 1], s_deg[kSnapNodes];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned full = 0xffffffffu;
+    for (int v = warp; v < n; v += 32) {  // a warp per variable: its neighbours, 32 words of the row at most
+        const uint32_t m = lane < W ? bits[(int64_t)v * W + lane] : 0u;
+        const int c = __popc(m);
+        int incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(full, incl, o);
+            if (lane >= o) incl += t;
+        }
+        int at = incl - c, higher = 0;
+        for (uint32_t r = m; r; r &= r - 1) {
+            const int u = lane * 32 + __ffs(r) - 1;
+            adjl[(int64_t)v * stride + at++] = u;
+            higher += u > v;
+        }
+        const int all = __shfl_sync(full, incl, 31);
+        higher = __reduce_add_sync(full, higher);
+        if (lane == 0) {
+            s_deg[v] = all;
+            deg[v] = all;
+            s_higher[v] = higher;
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {  // exclusive offsets of the variables' edges
+        int run = 0;
+        for (int v0 = 0; v0 < n; v0 += 32) {
+            const int h = v0 + lane < n ? s_higher[v0 + lane] : 0;
+            int incl = h;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(full, incl, o);
+                if (lane >= o) incl += t;
+            }
+            if (v0 + lane < n) s_higher[v0 + lane] = run + incl - h;
+            run += __shfl_sync(full, incl, 31);
+        }
+        if (lane == 0) {
+            s_higher[n] = run;
+            level_init(ctl, stats, run);
+        }
+    }
+    __syncthreads();
+    for (int v = warp; v < n; v += 32) {
+        const int32_t *L = adjl + (int64_t)v * stride;
+        const int dv = s_deg[v], o0 = s_higher[v], k0 = dv - (s_higher[v + 1] - o0);
+        for (int k = k0 + lane; k < dv; k += 32) {
+            const int u = L[k], o = o0 + k - k0;
+            ex[o] = v;
+            ey[o] = u;
+            pxy[o] = k;
+            pyx[o] = find_pos(adjl + (int64_t)u * stride, s_deg[u], v);
+            const uint64_t cx = sat_binom(btab, dv - 1, d, &stats[ST_UNSUPPORTED]);
+            const uint64_t cy = sat_binom(btab, s_deg[u] - 1, d, &stats[ST_UNSUPPORTED]);
+            cntx[o] = cx;
+            total[o] = cx + cy;
+            next[o] = 0;
+            status[o] = (cx + cy) == 0 ? kStatusKept : kStatusActive;
+        }
+    }
 }
 
 // Level 0 from the tensor-core Gram matrix (gram.cu): one warp per pair x < y (at level 0
@@ -783,6 +945,7 @@ extern "C" int fpgm_engine_create(int32_t device, fpgm_engine **out) {
     RET(e->btab.ensure(bt.size() * 8));
     CK(cudaMemcpy(e->btab.p, bt.data(), bt.size() * 8, cudaMemcpyHostToDevice));
     RET(e->counters.ensure(kCounterBytes));
+    CK(cudaHostAlloc(reinterpret_cast<void **>(&e->level_host), 1024, cudaHostAllocDefault));
     RET(e->stats.ensure(ST_COUNT * 8));
     e->wave_log = getenv("FPGM_WAVE_LOG") != nullptr;
     if (const char *pm = getenv("FPGM_PART_MAX_LOG")) e->part_max_log = std::min(kPartMaxLog, std::max(1, atoi(pm)));
@@ -843,6 +1006,7 @@ extern "C" int fpgm_engine_destroy(fpgm_engine *e) {
                       &e->strata_refs, &e->strata_used};
     for (DevBuf *b : bufs) b->release();
     gram_destroy(e->gram);
+    if (e->level_host) cudaFreeHost(e->level_host);
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->ev1) cudaEventDestroy(e->ev1);
     if (e->ev2) cudaEventDestroy(e->ev2);
@@ -1177,7 +1341,7 @@ void strata_args(fpgm_engine *e, StrataArgs &s) {
 
 // Level d's waves count through shared strata when a test can go past shared memory: buffers
 // made (or, when the last level came near their end, grown and emptied).  No room: not used.
-int strata_setup(fpgm_engine *e, int d, bool first) {
+int strata_setup(fpgm_engine *e, int d, bool first, const unsigned long long *last_used) {
     e->strata_level = false;
     if (first) e->strata_ready = false;
     if (!e->strata_on || !e->wide_on || e->wave_log || e->phase_timers.p || e->fixed_n < e->S || d < 1 ||
@@ -1185,11 +1349,8 @@ int strata_setup(fpgm_engine *e, int d, bool first) {
         return FPGM_OK;
     const size_t tab = kStrataKeyBytes + (size_t)kStrataNodes * 24 + (size_t)kStrataPairs * 16;
     const size_t slot = (size_t)((e->S + 15) & ~(int64_t)15) * 2;
-    unsigned long long used[3] = {0, 0, 0};
-    if (e->strata_ready) {
-        CK(cudaMemcpyAsync(used, e->strata_used.p, sizeof used, cudaMemcpyDeviceToHost, e->stream));
-        CK(cudaStreamSynchronize(e->stream));
-    }
+    unsigned long long used[3] = {0, 0, 0};  // at the end of the last level
+    if (e->strata_ready) memcpy(used, last_used, sizeof used);
     bool empty = !e->strata_ready;
     const size_t least = std::max<size_t>((size_t)256 << 20, slot * 8192);
     size_t want = std::max(least, e->strata_pool.bytes);
@@ -1376,13 +1537,70 @@ int launch_tiers(fpgm_engine *e, const WaveArgs &a) {
     return n;
 }
 
-// One level's waves driven by the device: a CUDA graph whose WHILE conditional node runs the
-// wave body (prep, plan, scan, classify, the counting tiers, reduce) until the tail kernel
-// finds no unresolved edge.  The graph is captured and instantiated once per level (the
-// level's edge count, |Z| and buffers are its parameters) and the host waits once per level.
-int run_waves_graph(fpgm_engine *e, double alpha, int d, int64_t n_active, fpgm_pc_stats *st, int level_idx,
-                    const WaveArgs &proto) {
+// What a level leaves for the host, copied once at its end.
+struct LevelHost {
+    unsigned long long stats[ST_COUNT], live[2], sets_used, strata_used[3];
+    WaveCtl ctl;
+};
+// A level whose waves are enqueued and not yet waited for.
+static_assert(sizeof(LevelHost) <= 1024, "the engine's pinned block");
+struct PendingLevel {
+    bool device = false, gram = false;  // device-driven waves / level 0 on the tensor cores
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    int per_wave = 0, launches = 0;
+    ~PendingLevel() {
+        if (exec) cudaGraphExecDestroy(exec);
+        if (graph) cudaGraphDestroy(graph);
+    }
+};
+
+// One wave on the current stream, from the edges' shares to their reduction.  Returns launches.
+int launch_wave(fpgm_engine *e, const WaveArgs &a, int64_t n_active, int in_graph, cudaGraphConditionalHandle h) {
     unsigned long long *dstat = e->stats.as<unsigned long long>();
+    WaveCtl *ctl = e->wave_ctl.as<WaveCtl>();
+    StrataArgs sa;
+    strata_args(e, sa);
+    StrataCounters *sc = a.strata_card ? sa.sc : nullptr;
+    int n = 3;  // classify, reduce, begin or prep
+    if (n_active <= kBeginEdges) {
+        wave_begin_kernel<<<1, 1024, 0, e->stream>>>(ctl, dstat, e->counters.as<int32_t>(), sc, (int)n_active,
+                                                     e->status.as<uint8_t>(), e->total.as<uint64_t>(),
+                                                     e->next.as<uint64_t>(), e->off.as<int32_t>(),
+                                                     (long long)e->ci_blocks, (long long)kMaxItems);
+    } else {
+        wave_prep_kernel<<<1, 128, 0, e->stream>>>(ctl, dstat, e->counters.as<int32_t>(), sc, (long long)n_active,
+                                                   (long long)e->ci_blocks, (long long)kMaxItems);
+        wave_plan_dev_kernel<<<blocks_for(n_active + 1, 256), 256, 0, e->stream>>>(
+            (int)n_active, e->status.as<uint8_t>(), e->total.as<uint64_t>(), e->next.as<uint64_t>(), ctl,
+            e->g.as<int32_t>());
+        size_t sb = e->scan_tmp.bytes;
+        cub::DeviceScan::ExclusiveSum(e->scan_tmp.p, sb, e->g.as<int32_t>(), e->off.as<int32_t>(),
+                                      (int)(n_active + 1), e->stream);
+        wave_stamp_kernel<<<1, 1, 0, e->stream>>>(ctl, -1);
+        n += 2;
+    }
+    classify_kernel<SRC_WAVE><<<e->ci_blocks, kThreads, 0, e->stream>>>(a);
+    n += launch_shared_tiers(e, a);
+    if (a.slot_mem) {
+        wave_stamp_kernel<<<1, 1, 0, e->stream>>>(ctl, 0);
+        if (a.strata_card) n += launch_strata(e, a);
+        n += 1 + launch_compact(e, a, e->n_slots);
+    }
+    wave_reduce_kernel<<<reduce_blocks(n_active, e->num_sms), 256, 0, e->stream>>>(
+        (int)n_active, e->off.as<int32_t>(), e->flag.as<uint8_t>(), e->status.as<uint8_t>(), e->next.as<uint64_t>(),
+        e->total.as<uint64_t>(), e->seprank.as<uint64_t>(), dstat, ctl, a.slot_mem != nullptr, in_graph, h);
+    return n;
+}
+
+// One level's waves driven by the device: a CUDA graph whose WHILE conditional node runs the
+// wave body until its reduction finds no unresolved edge.  The graph is captured and
+// instantiated once per level (the level's edge count, |Z| and buffers are its parameters).  A
+// level that one wave is sure to finish (no edge has more ranks than the first wave takes) is
+// launched without a graph, whose capture and launch would take longer than its kernels.
+// Nothing waits here: the host waits once per level, after its end has been enqueued too.
+int run_waves_graph(fpgm_engine *e, double alpha, int d, int64_t n_active, int64_t most_ranks, fpgm_pc_stats *st,
+                    const WaveArgs &proto, PendingLevel &pend) {
     // items of one wave at most
     const int64_t cap = std::max<int64_t>(n_active, std::min<int64_t>(kMaxItems, std::max<int64_t>(e->level_tests, 1 << 16)));
     WaveArgs a = proto;
@@ -1399,23 +1617,26 @@ int run_waves_graph(fpgm_engine *e, double alpha, int d, int64_t n_active, fpgm_
     a.off = e->off.as<int32_t>();
     a.n_edges = (int32_t)n_active;
     a.dbg = nullptr;
-    size_t sb = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, sb, e->g.as<int32_t>(), e->off.as<int32_t>(), (int)(n_active + 1),
-                                  e->stream);
-    RET(e->scan_tmp.ensure(sb + 16));
-    sb = e->scan_tmp.bytes;
-    RET(e->wave_ctl.ensure(sizeof(WaveCtl)));
-    WaveCtl *ctl = e->wave_ctl.as<WaveCtl>();
-    wave_ctl_init_kernel<<<1, 1, 0, e->stream>>>(ctl, dstat, (long long)n_active);
-    CK(cudaGetLastError());
+    if (n_active > kBeginEdges) {
+        size_t sb = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, sb, e->g.as<int32_t>(), e->off.as<int32_t>(), (int)(n_active + 1),
+                                      e->stream);
+        RET(e->scan_tmp.ensure(sb + 16));
+    }
+    pend.device = true;
+    // the first wave's share of every edge (wave_begin's rule; edges without ranks only raise it)
+    const int64_t q0 = std::min<int64_t>(std::min<int64_t>(4096, (e->ci_blocks * 64ll + n_active - 1) / n_active),
+                                         kMaxItems / n_active);
+    if (most_ranks <= q0) {
+        pend.per_wave = launch_wave(e, a, n_active, 0, cudaGraphConditionalHandle{});
+        CK(cudaGetLastError());
+        return FPGM_OK;
+    }
     const auto t0 = std::chrono::steady_clock::now();
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    int per_wave = 0;
     auto build = [&]() -> int {
-        CK(cudaGraphCreate(&graph, 0));
+        CK(cudaGraphCreate(&pend.graph, 0));
         cudaGraphConditionalHandle h;
-        CK(cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault));
+        CK(cudaGraphConditionalHandleCreate(&h, pend.graph, 1, cudaGraphCondAssignDefault));
         alignas(cudaGraphNodeParams) unsigned char cp_raw[sizeof(cudaGraphNodeParams)] = {};
         cudaGraphNodeParams &cp = *reinterpret_cast<cudaGraphNodeParams *>(cp_raw);
         cp.type = cudaGraphNodeTypeConditional;
@@ -1423,74 +1644,85 @@ int run_waves_graph(fpgm_engine *e, double alpha, int d, int64_t n_active, fpgm_
         cp.conditional.type = cudaGraphCondTypeWhile;
         cp.conditional.size = 1;
         cudaGraphNode_t cn;
-        CK(cudaGraphAddNode(&cn, graph, nullptr, nullptr, 0, &cp));
+        CK(cudaGraphAddNode(&cn, pend.graph, nullptr, nullptr, 0, &cp));
         cudaGraph_t body = cp.conditional.phGraph_out[0];
         CK(cudaStreamBeginCaptureToGraph(e->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-        StrataArgs sa;
-        strata_args(e, sa);
-        wave_prep_kernel<<<1, 32, 0, e->stream>>>(ctl, dstat, e->counters.as<int32_t>(),
-                                                  a.strata_card ? sa.sc : nullptr, (long long)n_active,
-                                                  (long long)e->ci_blocks, (long long)kMaxItems);
-        wave_plan_dev_kernel<<<blocks_for(n_active + 1, 256), 256, 0, e->stream>>>(
-            (int)n_active, e->status.as<uint8_t>(), e->total.as<uint64_t>(), e->next.as<uint64_t>(), ctl,
-            e->g.as<int32_t>());
-        cub::DeviceScan::ExclusiveSum(e->scan_tmp.p, sb, e->g.as<int32_t>(), e->off.as<int32_t>(),
-                                      (int)(n_active + 1), e->stream);
-        wave_stamp_kernel<<<1, 1, 0, e->stream>>>(ctl, -1);
-        classify_kernel<SRC_WAVE><<<e->ci_blocks, kThreads, 0, e->stream>>>(a);
-        per_wave = 8 + launch_shared_tiers(e, a);  // prep, plan, 3 stamps, classify, reduce, tail (+ tier 2)
-        wave_stamp_kernel<<<1, 1, 0, e->stream>>>(ctl, 0);
-        if (a.strata_card) per_wave += launch_strata(e, a);
-        if (a.slot_mem) per_wave += launch_compact(e, a, e->n_slots);
-        wave_stamp_kernel<<<1, 1, 0, e->stream>>>(ctl, 1);
-        wave_reduce_kernel<<<reduce_blocks(n_active, e->num_sms), 256, 0, e->stream>>>(
-            (int)n_active, e->off.as<int32_t>(), e->flag.as<uint8_t>(), e->status.as<uint8_t>(),
-            e->next.as<uint64_t>(), e->total.as<uint64_t>(), e->seprank.as<uint64_t>(), dstat);
-        wave_tail_kernel<<<1, 1, 0, e->stream>>>(ctl, dstat, h);
+        pend.per_wave = launch_wave(e, a, n_active, 1, h);
         const cudaError_t le = cudaGetLastError();
         const cudaError_t ce = cudaStreamEndCapture(e->stream, &body);
         if (le != cudaSuccess) return set_error(FPGM_ERR_CUDA, "level %d graph capture: %s", d, cudaGetErrorString(le));
         CK(ce);
-        CK(cudaGraphInstantiate(&exec, graph, 0));
+        CK(cudaGraphInstantiate(&pend.exec, pend.graph, 0));
         return FPGM_OK;
     };
-    int rc = build();
+    RET(build());
     st->graph_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-    if (rc == FPGM_OK) {
-        const cudaError_t le = cudaGraphLaunch(exec, e->stream);
-        if (le != cudaSuccess) rc = set_error(FPGM_ERR_CUDA, "cudaGraphLaunch: %s", cudaGetErrorString(le));
-    }
-    WaveCtl hc;
-    unsigned long long hs[ST_COUNT];
-    if (rc == FPGM_OK) {
-        cudaError_t ce = cudaMemcpyAsync(&hc, ctl, sizeof hc, cudaMemcpyDeviceToHost, e->stream);
-        if (ce == cudaSuccess) ce = cudaMemcpyAsync(hs, dstat, sizeof hs, cudaMemcpyDeviceToHost, e->stream);
-        if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
-        if (ce != cudaSuccess) rc = set_error(FPGM_ERR_CUDA, "level %d graph: %s", d, cudaGetErrorString(ce));
-    }
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-    if (rc != FPGM_OK) return rc;
-    if (hs[ST_UNSUPPORTED])
-        return set_error(FPGM_ERR_UNSUPPORTED,
-                         "level %d: %llu CI test(s) are outside the engine's limits (joint table beyond 2^62 "
-                         "cells or a node degree >= %d)",
-                         d, hs[ST_UNSUPPORTED], kBinomN);
-    if (hs[ST_UNRESOLVED]) return set_error(FPGM_ERR_STATE, "level %d: wave limit reached with edges unresolved", d);
-    st->waves[level_idx] = (int32_t)hc.n_waves;
-    st->count_ms += hc.count_ns / 1e6;
-    st->large_ms += hc.large_ns / 1e6;
-    st->count_bytes += (double)hs[ST_BYTES_SHARED];
-    st->large_bytes += (double)hs[ST_BYTES_LARGE];
-    st->count_launches += hc.n_waves;
-    st->kernel_launches += 1 + hc.n_waves * per_wave;  // + the control-block init
+    CK(cudaGraphLaunch(pend.exec, e->stream));
     return FPGM_OK;
 }
 
+// Level 0 of one dataset on the tensor cores: one rank per pair, at its own place.
+int enqueue_gram_level(fpgm_engine *e, double alpha, int64_t n_active, const WaveArgs &proto, PendingLevel &pend) {
+    unsigned long long *dstat = e->stats.as<unsigned long long>();
+    WaveArgs a = proto;
+    RET(wave_args_base(e, a, alpha, 0, n_active));
+    a.ex = proto.ex;
+    a.ey = proto.ey;
+    a.n_edges = (int32_t)n_active;
+    CK(cudaEventRecord(e->ev0, e->stream));
+    int nl = 0;
+    RET(gram_run(e->gram, e->stream, dstat + ST_TIMEOUT, &nl));
+    const int slice = gram_slice_ints(e->gram);
+    level0_gram_score_kernel<<<e->num_sms * e->gram_score_ctas, kThreads, kWarps * slice * 4, e->stream>>>(
+        a, gram_counts(e->gram), gram_ld(e->gram), gram_row_off(e->gram), (int)n_active, slice);
+    CK(cudaGetLastError());
+    CK(cudaEventRecord(e->ev1, e->stream));
+    wave_reduce_kernel<<<reduce_blocks(n_active, e->num_sms), 256, 0, e->stream>>>(
+        (int)n_active, nullptr, e->flag.as<uint8_t>(), e->status.as<uint8_t>(), e->next.as<uint64_t>(),
+        e->total.as<uint64_t>(), e->seprank.as<uint64_t>(), dstat, nullptr, 0, 0, cudaGraphConditionalHandle{});
+    CK(cudaGetLastError());
+    pend.gram = true;
+    pend.launches = nl + 2;
+    return FPGM_OK;
+}
+
+int unsupported_tests(int d, unsigned long long n) {
+    return set_error(FPGM_ERR_UNSUPPORTED,
+                     "level %d: %llu CI test(s) are outside the engine's limits (joint table beyond 2^62 "
+                     "cells or a node degree >= %d)",
+                     d, n, kBinomN);
+}
+
+// What a pending level's waves did, once the host has waited.
+int settle_level(fpgm_engine *e, int d, int64_t n_active, const PendingLevel &pend, const LevelHost &h, fpgm_pc_stats *st) {
+    if (pend.gram) {
+        float ms = 0.f;
+        CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
+        st->gram_ms += ms;
+        st->gram_flops += gram_flops(e->gram);
+        st->gram_tests += n_active;
+        st->kernel_launches += pend.launches;
+        st->waves[st->n_levels] = 1;
+        if (h.stats[ST_TIMEOUT])
+            return set_error(FPGM_ERR_TIMEOUT, "level %d: a bounded wait of the tensor-core level-0 kernel gave up", d);
+        return FPGM_OK;
+    }
+    if (!pend.device) return FPGM_OK;
+    if (h.stats[ST_UNSUPPORTED]) return unsupported_tests(d, h.stats[ST_UNSUPPORTED]);
+    if (h.stats[ST_UNRESOLVED]) return set_error(FPGM_ERR_STATE, "level %d: wave limit reached with edges unresolved", d);
+    st->waves[st->n_levels] = (int32_t)h.ctl.n_waves;
+    st->count_ms += h.ctl.count_ns / 1e6;
+    st->large_ms += h.ctl.large_ns / 1e6;
+    st->count_bytes += (double)h.stats[ST_BYTES_SHARED];
+    st->large_bytes += (double)h.stats[ST_BYTES_LARGE];
+    st->count_launches += h.ctl.n_waves;
+    st->kernel_launches += h.ctl.n_waves * pend.per_wave;
+    return FPGM_OK;
+}
+
+// One level's waves driven by the host (several datasets' level 0, FPGM_GRAPH=0, the wave log).
 int run_waves_and_count(fpgm_engine *e, double alpha, int d, int64_t n_active, fpgm_pc_stats *st, int level_idx,
-                        const WaveArgs &proto, bool gram = false) {
-    if (d >= 1 && e->graph_on && !e->wave_log && !e->phase_timers.p)
-        return run_waves_graph(e, alpha, d, n_active, st, level_idx, proto);
+                        const WaveArgs &proto) {
     unsigned long long *dstat = e->stats.as<unsigned long long>();
     int wave = 0;
     int64_t unresolved = n_active;
@@ -1528,28 +1760,18 @@ int run_waves_and_count(fpgm_engine *e, double alpha, int d, int64_t n_active, f
         a.off = e->off.as<int32_t>();
         a.n_edges = (int32_t)n_active;
         CK(cudaEventRecord(e->ev0, e->stream));
-        if (gram) {  // level 0: every pair's table from the tensor-core Gram matrix (one wave, one test per edge)
-            int nl = 0;
-            RET(gram_run(e->gram, e->stream, dstat + ST_TIMEOUT, &nl));
-            const int slice = gram_slice_ints(e->gram);
-            level0_gram_score_kernel<<<e->num_sms * e->gram_score_ctas, kThreads, kWarps * slice * 4, e->stream>>>(
-                a, gram_counts(e->gram), gram_ld(e->gram), gram_row_off(e->gram), (int)n_active, slice);
-            CK(cudaGetLastError());
-            st->kernel_launches += nl + 3;  // plan, one-hot + GEMM, scoring, reduce
-        } else {
-            classify_kernel<SRC_WAVE><<<e->ci_blocks, kThreads, 0, e->stream>>>(a);
-            st->kernel_launches += 3 + launch_shared_tiers(e, a);  // plan, classify, reduce
-            CK(cudaGetLastError());
-        }
+        classify_kernel<SRC_WAVE><<<e->ci_blocks, kThreads, 0, e->stream>>>(a);
+        st->kernel_launches += 3 + launch_shared_tiers(e, a);  // plan, classify, reduce
+        CK(cudaGetLastError());
         CK(cudaEventRecord(e->ev1, e->stream));
         a.dbg = e->phase_timers.as<unsigned long long>();
-        if (a.strata_card && !gram) {
+        if (a.strata_card) {
             StrataArgs sa;
             strata_args(e, sa);
             CK(cudaMemsetAsync(sa.sc, 0, sizeof(StrataCounters), e->stream));
             st->kernel_launches += launch_strata(e, a);
         }
-        if (a.slot_mem && !gram) {
+        if (a.slot_mem) {
             st->kernel_launches += launch_compact(e, a, e->n_slots);
             CK(cudaGetLastError());
         }
@@ -1586,7 +1808,8 @@ int run_waves_and_count(fpgm_engine *e, double alpha, int d, int64_t n_active, f
         CK(cudaMemsetAsync(dstat + ST_UNRESOLVED, 0, 8, e->stream));
         wave_reduce_kernel<<<reduce_blocks(n_active, e->num_sms), 256, 0, e->stream>>>(
             (int)n_active, e->off.as<int32_t>(), e->flag.as<uint8_t>(), e->status.as<uint8_t>(),
-            e->next.as<uint64_t>(), e->total.as<uint64_t>(), e->seprank.as<uint64_t>(), dstat);
+            e->next.as<uint64_t>(), e->total.as<uint64_t>(), e->seprank.as<uint64_t>(), dstat, nullptr, 0, 0,
+            cudaGraphConditionalHandle{});
         CK(cudaGetLastError());
         unsigned long long hs[ST_COUNT];
         int32_t T = 0, tiers[C_COUNT];
@@ -1597,31 +1820,19 @@ int run_waves_and_count(fpgm_engine *e, double alpha, int d, int64_t n_active, f
         float ms = 0.f, ms2 = 0.f;
         CK(cudaEventElapsedTime(&ms, e->ev0, e->ev1));
         CK(cudaEventElapsedTime(&ms2, e->ev1, e->ev2));
-        if (gram) {
-            st->gram_ms += ms;
-            st->gram_flops += gram_flops(e->gram);
-            st->gram_tests += n_active;
-        } else {
-            st->count_ms += ms;
-        }
+        st->count_ms += ms;
         st->large_ms += ms2;
         // algorithmic bytes: (2 + d) columns of the test's samples per test, split by kernel
         st->count_bytes += (double)hs[ST_BYTES_SHARED];
         st->large_bytes += (double)hs[ST_BYTES_LARGE];
-        if (!gram) st->count_launches += 1;
-        if (hs[ST_TIMEOUT])
-            return set_error(FPGM_ERR_TIMEOUT, "level %d: a bounded wait of the tensor-core level-0 kernel gave up", d);
+        st->count_launches += 1;
         if (e->wave_log)
             fprintf(stderr,
                     "wave level=%d tests=%d tier0=%d tier1=%d tier2=%d (partitioned=%d parallel=%d retried=%d) "
                     "compact_launched=%d count_ms=%.4f compact_ms=%.4f count_bytes=%.0f compact_bytes=%.0f\n",
                     d, T, tiers[C_TIER0], tiers[C_TIER1], tiers[C_TIER2], tiers[C_PART], tiers[C_WIDET], tiers[C_RETRY],
                     a.slot_mem != nullptr, ms, ms2, (double)hs[ST_BYTES_SHARED], (double)hs[ST_BYTES_LARGE]);
-        if (hs[ST_UNSUPPORTED])
-            return set_error(FPGM_ERR_UNSUPPORTED,
-                             "level %d: %llu CI test(s) are outside the engine's limits (joint table beyond 2^62 "
-                             "cells or a node degree >= %d)",
-                             d, hs[ST_UNSUPPORTED], kBinomN);
+        if (hs[ST_UNSUPPORTED]) return unsupported_tests(d, hs[ST_UNSUPPORTED]);
         unresolved = (int64_t)hs[ST_UNRESOLVED];
         ++wave;
     }
@@ -1680,13 +1891,28 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
         if (d > kMaxCond)
             return set_error(FPGM_ERR_UNSUPPORTED, "conditioning sets beyond %d variables are not supported",
                              kMaxCond);
-        int64_t n_active;
+        const bool complete = d == 0 && e->n_jobs == 1;  // level 0 of one dataset: every pair
+        const int64_t n_active = d == 0 ? E : (int64_t)st->edges_after[st->n_levels - 1];
+        const bool snap = !complete && d >= 1 && n <= kSnapNodes;  // the level's start in one launch
         int stride = 1;
-        if (d == 0 && e->n_jobs == 1) {
-            n_active = E;
-        } else {  // the level's snapshot (several datasets: also at level 0)
+        const size_t ne = (size_t)std::max<int64_t>(n_active, 1) + 1;
+        RET(e->edges_x.ensure(ne * 4));
+        RET(e->edges_y.ensure(ne * 4));
+        RET(e->pxy.ensure(ne * 4));
+        RET(e->pyx.ensure(ne * 4));
+        RET(e->cntx.ensure(ne * 8));
+        RET(e->total.ensure(ne * 8));
+        RET(e->next.ensure(ne * 8));
+        RET(e->seprank.ensure(ne * 8));
+        RET(e->status.ensure(ne));
+        RET(e->g.ensure(ne * 4));
+        RET(e->off.ensure(ne * 4));
+        RET(e->wave_ctl.ensure(sizeof(WaveCtl)));
+        if (!complete) {  // the level's snapshot (several datasets: also at level 0)
             stride = std::max(1, max_deg);
             RET(e->adjl.ensure((size_t)n * stride * 4));
+        }
+        if (!complete && !snap) {
             csr_kernel<<<blocks_for(n, 128), 128, 0, e->stream>>>(e->bits.as<uint32_t>(), n, W, e->adjl.as<int32_t>(),
                                                                  stride, e->deg.as<int32_t>(),
                                                                  e->node_cnt.as<int32_t>());
@@ -1700,25 +1926,10 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
             sb = e->scan_tmp.bytes;
             CK(cub::DeviceScan::ExclusiveSum(e->scan_tmp.p, sb, e->node_cnt.as<int32_t>(), e->node_off.as<int32_t>(),
                                              n + 1, e->stream));
-            int32_t na = 0;
-            CK(cudaMemcpyAsync(&na, e->node_off.as<int32_t>() + n, 4, cudaMemcpyDeviceToHost, e->stream));
-            CK(cudaStreamSynchronize(e->stream));
-            n_active = na;
         }
-        const size_t ne = (size_t)std::max<int64_t>(n_active, 1) + 1;
-        RET(e->edges_x.ensure(ne * 4));
-        RET(e->edges_y.ensure(ne * 4));
-        RET(e->pxy.ensure(ne * 4));
-        RET(e->pyx.ensure(ne * 4));
-        RET(e->cntx.ensure(ne * 8));
-        RET(e->total.ensure(ne * 8));
-        RET(e->next.ensure(ne * 8));
-        RET(e->seprank.ensure(ne * 8));
-        RET(e->status.ensure(ne));
-        RET(e->g.ensure(ne * 4));
-        RET(e->off.ensure(ne * 4));
+        PendingLevel pend;
         if (n_active > 0) {
-            if (d == 0 && e->n_jobs == 1) {
+            if (complete) {
                 level0_edges_kernel<<<blocks_for(E, 256), 256, 0, e->stream>>>(
                     n, e->edges_x.as<int32_t>(), e->edges_y.as<int32_t>(), e->pxy.as<int32_t>(),
                     e->pyx.as<int32_t>(), e->cntx.as<uint64_t>(), e->total.as<uint64_t>(), e->next.as<uint64_t>(),
@@ -1729,6 +1940,12 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
                     e->edges_x.as<int32_t>(), e->edges_y.as<int32_t>(), e->pxy.as<int32_t>(), e->pyx.as<int32_t>(),
                     e->cntx.as<uint64_t>(), e->total.as<uint64_t>(), e->next.as<uint64_t>(),
                     e->status.as<uint8_t>());
+            } else if (snap) {
+                level_snapshot_kernel<<<1, 1024, 0, e->stream>>>(
+                    e->bits.as<uint32_t>(), n, W, d, e->adjl.as<int32_t>(), stride, e->deg.as<int32_t>(),
+                    e->btab.as<uint64_t>(), e->edges_x.as<int32_t>(), e->edges_y.as<int32_t>(), e->pxy.as<int32_t>(),
+                    e->pyx.as<int32_t>(), e->cntx.as<uint64_t>(), e->total.as<uint64_t>(), e->next.as<uint64_t>(),
+                    e->status.as<uint8_t>(), dstat, e->wave_ctl.as<WaveCtl>());
             } else {
                 level_edges_kernel<<<blocks_for(n, 128), 128, 0, e->stream>>>(
                     n, d, e->adjl.as<int32_t>(), stride, e->deg.as<int32_t>(), e->node_off.as<int32_t>(),
@@ -1738,7 +1955,13 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
             }
             CK(cudaGetLastError());
             st->kernel_launches += 1;
-            CK(cudaMemsetAsync(dstat + ST_DET, 0, 8 * 2, e->stream));
+        }
+        if (!snap || n_active == 0) {
+            level_init_kernel<<<1, 1, 0, e->stream>>>(e->wave_ctl.as<WaveCtl>(), dstat, (long long)n_active);
+            CK(cudaGetLastError());
+            st->kernel_launches += 1;
+        }
+        if (n_active > 0) {
             WaveArgs a;
             memset(&a, 0, sizeof a);
             a.adjl = e->adjl.as<int32_t>();
@@ -1772,55 +1995,67 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
                                 e->pair_g2.ensure((size_t)n * n * sizeof(float)) == FPGM_OK;
             }
             if (!gram) RET(live_setup(e, d));
-            {  // a test per rank: at most C(max_deg - 1, d) from either side of an edge
-                double c = 2.0 * (double)n_active;
-                for (int k = 0; k < d; ++k) c = std::min(1e15, c * std::max(0, max_deg - 1 - k) / (k + 1));
-                e->level_tests = d == 0 ? n_active : (int64_t)c + 64;
-            }
+            // a test per rank: at most C(max_deg - 1, d) from either side of an edge
+            double ranks = 2.0;
+            for (int k = 0; k < d; ++k) ranks = std::min(1e15, ranks * std::max(0, max_deg - 1 - k) / (k + 1));
+            e->level_tests = d == 0 ? n_active : (int64_t)std::min(1e15, ranks * (double)n_active) + 64;
             if (!gram) RET(sets_setup(e, d, n_active));
             if (d == 0 && !gram && !(e->sets_level && e->sets_all)) e->pairs_kept = false;  // some tests count their own
-            RET(strata_setup(e, d, d <= 1));
-            RET(run_waves_and_count(e, alpha, d, n_active, st, st->n_levels, a, gram));
-            if (e->live_on && e->live_stat.p) {
-                // Bitmaps pay for themselves when the next level can leave enough samples out:
-                // the next level writes them when this one's partition-path tests had fewer than
-                // live_frac of their samples in contributing strata (the fraction falls with |Z|).
-                unsigned long long ls[2];
-                CK(cudaMemcpyAsync(ls, e->live_stat.p, 16, cudaMemcpyDeviceToHost, e->stream));
-                CK(cudaStreamSynchronize(e->stream));
-                const unsigned long long din = ls[0] - e->live_prev[0], dall = ls[1] - e->live_prev[1];
-                e->live_prev[0] = ls[0];
-                e->live_prev[1] = ls[1];
-                e->live_next = dall > 0 && (double)din < e->live_frac * (double)dall;
-                if (e->wave_log && dall > 0)
-                    fprintf(stderr, "live level=%d contributing=%.3f wrote=%d next_writes=%d\n", d,
-                            (double)din / (double)dall, (int)e->live_write, (int)e->live_next);
-            }
+            RET(strata_setup(e, d, d <= 1, e->level_host->strata_used));
+            if (gram)
+                RET(enqueue_gram_level(e, alpha, n_active, a, pend));
+            else if (d >= 1 && e->graph_on && !e->wave_log && !e->phase_timers.p)
+                RET(run_waves_graph(e, alpha, d, n_active, (int64_t)ranks + 1, st, a, pend));
+            else
+                RET(run_waves_and_count(e, alpha, d, n_active, st, st->n_levels, a));
         }
         // finalize: removals into the bitset and the removal log
         RET(e->log_vars.ensure((size_t)(var_count + std::max<int64_t>(n_active, 1) * std::max(d, 1)) * 4 + 16, true,
                                e->stream));
         if (var_count + n_active * (int64_t)d > INT32_MAX)
             return set_error(FPGM_ERR_UNSUPPORTED, "separating-set storage beyond 2^31 entries");
-        CK(cudaMemsetAsync(dstat + ST_REMOVED, 0, 16, e->stream));
+        const bool one = n_active <= 16384 && (int64_t)n * W <= 32768;  // removals and degrees in one CTA
         if (n_active > 0) {
-            level_finalize_kernel<<<blocks_for(n_active, 256), 256, 0, e->stream>>>(
+            level_finalize_kernel<<<one ? 1 : blocks_for(n_active, 256), one ? 1024 : 256, 0, e->stream>>>(
                 (int)n_active, d, W, e->edges_x.as<int32_t>(), e->edges_y.as<int32_t>(), e->pxy.as<int32_t>(),
                 e->pyx.as<int32_t>(), e->cntx.as<uint64_t>(), e->seprank.as<uint64_t>(), e->status.as<uint8_t>(),
                 e->adjl.as<int32_t>(), stride, e->deg.as<int32_t>(), e->btab.as<uint64_t>(), e->bits.as<uint32_t>(),
                 e->log_pair.as<int32_t>(), e->log_meta.as<int32_t>(), e->log_vars.as<int32_t>(), log_count, var_count,
-                dstat);
+                dstat, one, n);
             CK(cudaGetLastError());
             st->kernel_launches += 1;
         }
-        degree_kernel<<<blocks_for(n, 128), 128, 0, e->stream>>>(e->bits.as<uint32_t>(), n, W, dstat);
-        CK(cudaGetLastError());
-        st->kernel_launches += 1;
-        unsigned long long hs[ST_COUNT], h_sets_used = 0;
-        CK(cudaMemcpyAsync(hs, dstat, sizeof hs, cudaMemcpyDeviceToHost, e->stream));
-        if (e->sets_level) CK(cudaMemcpyAsync(&h_sets_used, e->set_tab.p, 8, cudaMemcpyDeviceToHost, e->stream));
+        if (!one || n_active == 0) {
+            degree_kernel<<<blocks_for(n, 128), 128, 0, e->stream>>>(e->bits.as<uint32_t>(), n, W, dstat);
+            CK(cudaGetLastError());
+            st->kernel_launches += 1;
+        }
+        LevelHost &h = *e->level_host;
+        CK(cudaMemcpyAsync(h.stats, dstat, sizeof h.stats, cudaMemcpyDeviceToHost, e->stream));
+        if (pend.device) CK(cudaMemcpyAsync(&h.ctl, e->wave_ctl.p, sizeof h.ctl, cudaMemcpyDeviceToHost, e->stream));
+        h.sets_used = 0;
+        if (e->sets_level) CK(cudaMemcpyAsync(&h.sets_used, e->set_tab.p, 8, cudaMemcpyDeviceToHost, e->stream));
+        h.strata_used[0] = h.strata_used[1] = h.strata_used[2] = 0;
+        if (e->strata_ready)
+            CK(cudaMemcpyAsync(h.strata_used, e->strata_used.p, sizeof h.strata_used, cudaMemcpyDeviceToHost, e->stream));
+        const bool live = n_active > 0 && e->live_on && e->live_stat.p;
+        if (live) CK(cudaMemcpyAsync(h.live, e->live_stat.p, 16, cudaMemcpyDeviceToHost, e->stream));
         CK(cudaStreamSynchronize(e->stream));
-        e->sets_used = h_sets_used;
+        RET(settle_level(e, d, n_active, pend, h, st));
+        if (live) {
+            // Bitmaps pay for themselves when the next level can leave enough samples out:
+            // the next level writes them when this one's partition-path tests had fewer than
+            // live_frac of their samples in contributing strata (the fraction falls with |Z|).
+            const unsigned long long din = h.live[0] - e->live_prev[0], dall = h.live[1] - e->live_prev[1];
+            e->live_prev[0] = h.live[0];
+            e->live_prev[1] = h.live[1];
+            e->live_next = dall > 0 && (double)din < e->live_frac * (double)dall;
+            if (e->wave_log && dall > 0)
+                fprintf(stderr, "live level=%d contributing=%.3f wrote=%d next_writes=%d\n", d,
+                        (double)din / (double)dall, (int)e->live_write, (int)e->live_next);
+        }
+        const unsigned long long *hs = h.stats;
+        e->sets_used = h.sets_used;
         const int64_t removed = (int64_t)hs[ST_REMOVED];
         log_count += removed;
         var_count += removed * d;
