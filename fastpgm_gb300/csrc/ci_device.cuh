@@ -353,12 +353,13 @@ struct Verdict {
     unsigned long long hash;
 };
 
-// Full scoring of a dense table held by group g (shared or global memory).
+// Full scoring of a dense table held by group g (shared or global memory).  want_p: the p-value
+// of a decided test too (a recheck has it).
 // Every thread of g calls it; the verdict is valid in the group's thread 0.
 template <class G>
 __device__ inline Verdict score_dense(const G &g, const int *ct, int *ni, int *nj, int *nk, int dx, int dy,
                                       int64_t dz, double alpha, const BandTables &bt, bool want_p, bool want_hash,
-                                      Partial *scratch) {
+                                      Partial *scratch, bool defer = false) {
     Partial p{0, 0.0, 0.0, 0.0, 0ull};
     p.df = marginals(g, ct, ni, nj, nk, dx, dy, dz);
     const int64_t cells = dz * dx * dy;
@@ -375,7 +376,9 @@ __device__ inline Verdict score_dense(const G &g, const int *ct, int *ni, int *n
         Partial r2 = group_sum(g, q, scratch);
         v.g2 = r2.g2;
         v.rechecked = 1;
-        if (g.t < 32) {
+        if (defer) {  // the caller's host evaluates p and decides; dp carries the FP32 statistic
+            v.dp = r.g2;
+        } else if (g.t < 32) {
             v.p = chisq_pvalue(g.t == 1 ? r.g2 : r2.g2, r.df);
             v.indep = v.p > alpha;
             v.dp = fabs(v.p - __shfl_sync(0xffffffffu, v.p, 1));

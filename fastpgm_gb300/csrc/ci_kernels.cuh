@@ -2984,12 +2984,20 @@ struct PlainArgs {
     double alpha;
     BandTables bt;
     int32_t want_hash;
-    int32_t *gtab;  // zeroed table + marginals
-    int32_t *done;  // ticket counter, reset by the last CTA
+    int32_t host_p;  // the host forms p (and a recheck's decision) from the statistic
+    int32_t *gtab;   // zeroed table + marginals
+    int32_t *done;   // ticket counter, reset by the last CTA
     fpgm_ci_result *out;
     unsigned long long *stats;
 };
 
+// One CTA's share of the samples goes into replicas of the table in shared memory; a lone CTA
+// scores from there, several add theirs into the global table and the last one takes it back
+// into its shared memory (when table and marginals fit) before scoring, so that the chain of
+// scoring steps waits for shared memory and not for L2.  With host_p no p-value is evaluated
+// here: 6 to 40 us of dependent FP64 on one thread, 1 us on the host.  Bound by the launch, the
+// latency of that chain and the wait; a call of 5,000 samples took 45.1 us and takes 24.5 us, of
+// 500,000 samples 44.6 and 30.3 us.
 __global__ void __launch_bounds__(kThreads) ci_plain_kernel(PlainArgs p) {
     extern __shared__ int smem[];
     __shared__ const uint8_t *s_col[kMaxCols];
@@ -3012,35 +3020,40 @@ __global__ void __launch_bounds__(kThreads) ci_plain_kernel(PlainArgs p) {
     const int64_t per = (nvec + gridDim.x - 1) / gridDim.x;
     const int64_t v0 = min(nvec, per * blockIdx.x), v1 = min(nvec, v0 + per);
     const bool tail = blockIdx.x == 0;
-    if (cells + marg <= kCtaInts && cells < 65536) {
-        const int stride = (int)cells | 1;
-        int R = 1;
-        for (int r = 32; r >= 2; r >>= 1)
-            if (stride * r <= kCtaInts) { R = r; break; }
-        for (int i = tid; i < stride * R; i += kThreads) smem[i] = 0;
+    const bool small = cells + marg <= kCtaInts && cells < 65536;  // table and marginals fit shared memory
+    int *ct = p.gtab;
+    if (small) {
+        // the replicas, then (a lone CTA) the summed table: as many replicas as leave it room
+        int lgR = 0;
+        while (lgR < 5 && (cells << (lgR + 1)) + cells + marg <= kCtaInts && (cells << (lgR + 3)) <= p.S) ++lgR;
+        const int R = 1 << lgR;
+        for (int i = tid; i < ((int)cells << lgR); i += kThreads) smem[i] = 0;
         __syncthreads();
-        int *mytab = smem + (lane & (R - 1)) * stride;
+        int *rep = smem + (lane & (R - 1));
         for (int64_t v = v0 + tid; v < v1; v += kThreads) {
             uint32_t c2[8] = {0, 0, 0, 0, 0, 0, 0, 0};
             for (int j = 0; j < ncols; ++j) horner16(c2, __ldg(reinterpret_cast<const uint4 *>(s_col[j]) + v), s_dim[j]);
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-                atomicAdd(&mytab[c2[q] & 0xffffu], 1);
-                atomicAdd(&mytab[c2[q] >> 16], 1);
+                atomicAdd(&rep[(c2[q] & 0xffffu) << lgR], 1);
+                atomicAdd(&rep[(c2[q] >> 16) << lgR], 1);
             }
         }
         if (tail)
             for (int64_t s = (p.S & ~(int64_t)15) + tid; s < p.S; s += kThreads) {
                 uint32_t c = 0;
                 for (int j = 0; j < ncols; ++j) c = c * s_dim[j] + s_col[j][s];
-                atomicAdd(&mytab[c], 1);
+                atomicAdd(&rep[c << lgR], 1);
             }
         __syncthreads();
+        int *sum = R > 1 ? smem + ((int)cells << lgR) : smem;
         for (int c = tid; c < (int)cells; c += kThreads) {
             int s = 0;
-            for (int r = 0; r < R; ++r) s += smem[r * stride + c];
-            if (s) atomicAdd(&p.gtab[c], s);
+            for (int r = 0; r < R; ++r) s += smem[(c << lgR) + ((r + tid) & (R - 1))];
+            if (gridDim.x == 1) sum[c] = s;
+            else if (s) atomicAdd(&p.gtab[c], s);
         }
+        ct = sum;
     } else {
         for (int64_t v = v0 * 16 + tid; v < v1 * 16; v += kThreads) {
             uint32_t c = 0;
@@ -3054,16 +3067,26 @@ __global__ void __launch_bounds__(kThreads) ci_plain_kernel(PlainArgs p) {
                 atomicAdd(&p.gtab[c], 1);
             }
     }
-    __threadfence();
+    if (gridDim.x > 1 || !small) {
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) s_last = atomicAdd(p.done, 1) == (int)gridDim.x - 1;
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        if (small) {
+            ct = smem;
+            for (int i = tid; i < (int)cells; i += kThreads) {
+                smem[i] = __ldcg(p.gtab + i);
+                p.gtab[i] = 0;  // the table is left zeroed
+            }
+        }
+    }
     __syncthreads();
-    if (tid == 0) s_last = atomicAdd(p.done, 1) == (int)gridDim.x - 1;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    int *ct = p.gtab;
     int *ni = ct + cells, *nj = ni + dz * dx, *nk = nj + dz * dy;
     const CtaGroup g{tid};
-    const Verdict v = score_dense(g, ct, ni, nj, nk, dx, dy, dz, p.alpha, p.bt, true, p.want_hash != 0, scratch);
+    const Verdict v = score_dense(g, ct, ni, nj, nk, dx, dy, dz, p.alpha, p.bt, !p.host_p, p.want_hash != 0, scratch,
+                                  p.host_p != 0);
     if (tid == 0) {
         fpgm_ci_result r;
         r.table_hash = p.want_hash ? table_hash(ct, cells) : 0;
@@ -3076,15 +3099,20 @@ __global__ void __launch_bounds__(kThreads) ci_plain_kernel(PlainArgs p) {
         r.rechecked = v.rechecked;
         r.path = 1;
         *p.out = r;
-        if (v.rechecked) {
+        if (p.host_p) {
+            *reinterpret_cast<double *>(p.out + 1) = v.dp;  // a recheck's FP32 statistic
+        } else if (v.rechecked) {
             atomicAdd(&p.stats[ST_RECHECK], 1ull);
             if (fabs(v.p - p.alpha) < 1e-12) atomicAdd(&p.stats[ST_NEARTIE], 1ull);
             atomicMax(&p.stats[ST_MAXDP], (unsigned long long)__double_as_longlong(v.dp));
         }
     }
-    __syncthreads();
-    for (int64_t i = tid; i < cells + marg; i += kThreads) ct[i] = 0;
-    if (tid == 0) *p.done = 0;
+    if (gridDim.x > 1 || !small) {
+        __syncthreads();
+        if (!small)
+            for (int64_t i = tid; i < cells + marg; i += kThreads) ct[i] = 0;
+        if (tid == 0) *p.done = 0;
+    }
 }
 
 }  // namespace fpgm

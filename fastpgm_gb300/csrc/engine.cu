@@ -1543,7 +1543,7 @@ struct LevelHost {
     WaveCtl ctl;
 };
 // A level whose waves are enqueued and not yet waited for.
-static_assert(sizeof(LevelHost) <= 1024, "the engine's pinned block");
+static_assert(sizeof(LevelHost) <= 512, "the engine's pinned block: a test's record follows");
 struct PendingLevel {
     bool device = false, gram = false;  // device-driven waves / level 0 on the tensor cores
     cudaGraph_t graph = nullptr;
@@ -2189,12 +2189,29 @@ int plain_test(fpgm_engine *e, int x, int y, const int *z, int d, double alpha, 
         p.bt.hi = p.bt.lo + e->band_df + 1;
         p.bt.dfmax = e->band_df;
         p.want_hash = want_hash;
+        p.host_p = 1;
         p.gtab = e->plain_ws.as<int32_t>();
         p.done = reinterpret_cast<int32_t *>(e->plain_ws.as<char>() + (size_t)kPlainInts * 4);
-        p.out = e->detail_buf.as<fpgm_ci_result>();
+        fpgm_ci_result *res = reinterpret_cast<fpgm_ci_result *>(reinterpret_cast<char *>(e->level_host) + 512);
+        p.out = res;  // pinned: the kernel writes the record where the host reads it
         p.stats = e->stats.as<unsigned long long>();
         ci_plain_kernel<<<plain_grid(e, p.S), kThreads, kSmemBytes, e->stream>>>(p);
         CK(cudaGetLastError());
+        if (st) st->kernel_launches += 1;
+        CK(cudaStreamSynchronize(e->stream));
+        *out = *res;
+        if (out->df > 0) out->p_value = chisq_pvalue(out->g2, out->df);
+        if (out->rechecked) {
+            double g32;
+            memcpy(&g32, res + 1, sizeof g32);
+            out->independent = out->p_value > alpha;
+            if (st) {
+                st->rechecks += 1;
+                st->near_ties += fabs(out->p_value - alpha) < 1e-12;
+                st->max_abs_dp = std::max(st->max_abs_dp, fabs(out->p_value - chisq_pvalue(g32, out->df)));
+            }
+        }
+        return FPGM_OK;
     } else {
         WaveArgs a;
         RET(wave_args_base(e, a, alpha, d, 1));
@@ -2316,10 +2333,12 @@ int run_plain(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
     unsigned long long hs[ST_COUNT];
     CK(cudaMemcpyAsync(hs, dstat, sizeof hs, cudaMemcpyDeviceToHost, e->stream));
     CK(cudaStreamSynchronize(e->stream));
-    st->rechecks = (int64_t)hs[ST_RECHECK];
-    st->near_ties = (int64_t)hs[ST_NEARTIE];
-    unsigned long long mdp = hs[ST_MAXDP];
-    memcpy(&st->max_abs_dp, &mdp, 8);
+    // tests beyond the plain kernel's table count on the device
+    st->rechecks += (int64_t)hs[ST_RECHECK];
+    st->near_ties += (int64_t)hs[ST_NEARTIE];
+    double dp;
+    memcpy(&dp, &hs[ST_MAXDP], 8);
+    st->max_abs_dp = std::max(st->max_abs_dp, dp);
     std::sort(rem.begin(), rem.end(), [](const Rem &p, const Rem &q) { return p.a != q.a ? p.a < q.a : p.b < q.b; });
     e->res_adj = adj;
     e->res_removed.clear();

@@ -1,0 +1,51 @@
+"""Dataset upload, parameter tables and single tests at the edges of their kernels' splits: first-
+appearance ids and cardinalities (one CTA or a cluster per column), parameter tables counted in
+one or several slices, and single tests on one or several CTAs.  The expected values are NumPy's
+and the oracle's; ids, counts and tables are compared exactly."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+import fastpgm_gb300 as F
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def eng():
+    e = F.Engine(0)
+    yield e
+    e.close()
+
+
+@pytest.mark.parametrize("S", [1, 15, 16, 4096, 8192, 40007])
+def test_single_tests(eng, S):
+    """fpgm_ci_test and its allocation-free form on one CTA and on several: counts, df and
+    decisions equal to the oracle's, G^2 and p within the FP32 screen's bounds."""
+    torch = pytest.importorskip("torch")
+    lib = F.load()
+    raw, _, _ = F.generate(n_nodes=10, n_samples=S, seed=17, n_edges=12, max_indegree=3, card=(2, 6))
+    card = eng.upload(raw)
+    cols = eng.download()
+    pitch = (S + 63) // 64 * 64
+    dev = torch.zeros((cols.shape[0], pitch), dtype=torch.uint8, device="cuda:0")
+    dev[:, :S] = torch.from_numpy(cols)
+    res = torch.zeros(ctypes.sizeof(F.CIResult), dtype=torch.uint8, device="cuda:0")
+    rng = np.random.default_rng(S)
+    for d in (0, 1, 2, 4):
+        t = [int(v) for v in rng.choice(cols.shape[0], size=2 + d, replace=False)]
+        want = O.ci_tests(cols, np.asarray(card, dtype=np.uint8), np.array([t], dtype=np.int32), d, threads=1)[0]
+        z = np.array(t[2:] or [0], dtype=np.int32)
+        rc = lib.fpgm_ci_test_noalloc(dev.data_ptr(), pitch, cols.shape[0], S, t[0], t[1],
+                                      z.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)), d, 0.05, 1, res.data_ptr(),
+                                      None)
+        assert rc == 0, lib.fpgm_last_error()
+        torch.cuda.synchronize()
+        for got in (F.CIResult.from_buffer_copy(res.cpu().numpy().tobytes()),
+                    eng.ci_test(t[0], t[1], t[2:], want_hash=True)):
+            assert got.table_hash == want.table_hash and got.cell_hash == want.cell_hash, t
+            assert got.df == want.df and got.independent == want.independent, t
+            assert abs(got.g2 - want.g2) <= max(2e-3, 2e-5 * abs(want.g2)), t
+            assert abs(got.p_value - want.p_value) <= (1e-10 if got.rechecked else 1e-3), t
