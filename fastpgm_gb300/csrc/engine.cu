@@ -15,6 +15,7 @@
 //     FreeDegree stop rule (:620-626, :387) is evaluated on the device.
 // Plain mode is the reference's control flow on the host with one kernel
 // launch (whole GPU) per CI test; it is the comparison baseline.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <cub/cub.cuh>
 
@@ -2637,7 +2638,8 @@ constexpr int kNoAllocMaxVars = 65536;
 constexpr int64_t kNoAllocDoneOff = kNoAllocTableInts;                    // ints
 constexpr int64_t kNoAllocCardOff = kNoAllocTableInts + 64;               // ints
 constexpr int64_t kNoAllocStatsOff = kNoAllocCardOff + kNoAllocMaxVars / 4;  // ints (8-byte aligned)
-constexpr int64_t kNoAllocInts = kNoAllocStatsOff + 2 * ST_COUNT + 64;
+constexpr int64_t kNoAllocPackedOff = kNoAllocStatsOff + 2 * ST_COUNT;  // cardinalities in test order, bytes
+constexpr int64_t kNoAllocInts = kNoAllocPackedOff + kMaxCols + 64;
 
 static __device__ __align__(256) int32_t g_noalloc_scratch[kNoAllocInts];
 
@@ -2649,18 +2651,38 @@ struct NoAllocDevice {
 std::mutex g_noalloc_mu;
 NoAllocDevice g_noalloc_dev[64];
 
-// Largest id + 1 of each listed column (the cardinality of dense ids).
-__global__ void noalloc_card_kernel(const uint8_t *columns, int64_t pitch, int64_t S, PlainArgs p, uint8_t *card) {
+// Largest id + 1 of each listed column (the cardinality of dense ids): a cluster of kCardSlices
+// CTAs per column, 16 samples a thread and load, the maxima met in the first CTA's shared memory
+// (nothing to clear beforehand, nothing left over for a later call). The counts go to `card` by
+// variable and to `packed` in test order for one copy to the host; what the counting kernel
+// expects to start at zero is cleared here. Bound by the latency of its loads: 4.4 us for 5 columns
+// of 50,000 samples (26.6 us with one CTA per column reading single bytes).
+constexpr int kCardSlices = 8;
+__global__ void __cluster_dims__(kCardSlices, 1, 1)
+    noalloc_card_kernel(const uint8_t *columns, int64_t pitch, int64_t S, PlainArgs p, uint8_t *card, uint8_t *packed,
+                        int32_t *done, unsigned long long *stats) {
     __shared__ unsigned s_max;
-    const int var = p.vars[blockIdx.x];
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int col = blockIdx.x / kCardSlices, slice = blockIdx.x % kCardSlices;
+    const uint8_t *c = columns + (int64_t)p.vars[col] * pitch;
     if (threadIdx.x == 0) s_max = 0;
-    __syncthreads();
-    const uint8_t *c = columns + (int64_t)var * pitch;
+    cluster.sync();
+    const int64_t nvec = S >> 4;
     unsigned m = 0;
-    for (int64_t s = threadIdx.x; s < S; s += blockDim.x) m = max(m, (unsigned)c[s]);
-    atomicMax(&s_max, m);
-    __syncthreads();
-    if (threadIdx.x == 0) card[var] = (uint8_t)(s_max + 1);
+    for (int64_t v = (int64_t)slice * blockDim.x + threadIdx.x; v < nvec; v += kCardSlices * blockDim.x) {
+        const uint4 w = __ldg(reinterpret_cast<const uint4 *>(c) + v);
+        m = __vmaxu4(m, __vmaxu4(__vmaxu4(w.x, w.y), __vmaxu4(w.z, w.w)));
+    }
+    unsigned b = max(max(m & 0xffu, (m >> 8) & 0xffu), max((m >> 16) & 0xffu, m >> 24));
+    if (slice == 0)
+        for (int64_t s = (S & ~(int64_t)15) + threadIdx.x; s < S; s += blockDim.x) b = max(b, (unsigned)c[s]);
+    b = __reduce_max_sync(0xffffffffu, b);
+    if ((threadIdx.x & 31) == 0) atomicMax(cluster.map_shared_rank(&s_max, 0), b);
+    cluster.sync();
+    if (slice != 0) return;
+    if (threadIdx.x == 0) packed[col] = card[p.vars[col]] = (uint8_t)(s_max + 1);  // 256 wraps to 0
+    if (col == 0 && threadIdx.x < ST_COUNT) stats[threadIdx.x] = 0;
+    if (col == 0 && threadIdx.x == 0) *done = 0;
 }
 
 // Per device, with that device current: resolve the scratch array's device
@@ -2718,11 +2740,13 @@ extern "C" int fpgm_ci_test_noalloc(const uint8_t *columns, int64_t pitch, int32
     p.vars[nz] = x;
     p.vars[nz + 1] = y;
     // cardinalities of the involved columns, then the size check on the host
-    noalloc_card_kernel<<<p.ncols, 256, 0, st>>>(columns, pitch, n_samples, p, card);
+    uint8_t *packed = reinterpret_cast<uint8_t *>(scratch + kNoAllocPackedOff);
+    noalloc_card_kernel<<<p.ncols * kCardSlices, 256, 0, st>>>(
+        columns, pitch, n_samples, p, card, packed, scratch + kNoAllocDoneOff,
+        reinterpret_cast<unsigned long long *>(scratch + kNoAllocStatsOff));
     CK(cudaGetLastError());
     uint8_t hc[kMaxCols];
-    for (int k = 0; k < p.ncols; ++k)
-        CK(cudaMemcpyAsync(&hc[k], card + p.vars[k], 1, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(hc, packed, p.ncols, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     for (int k = 0; k < p.ncols; ++k)
         if (hc[k] == 0)
@@ -2736,10 +2760,6 @@ extern "C" int fpgm_ci_test_noalloc(const uint8_t *columns, int64_t pitch, int32
                          "fpgm_ci_test_noalloc: the test needs %.0f table ints, beyond the fixed scratch of %lld; use "
                          "fpgm_ci_test, which allocates",
                          need, (long long)kNoAllocTableInts);
-    // the scratch keeps the previous call's contents: clear what must start at zero
-    CK(cudaMemsetAsync(scratch, 0, (size_t)need * 4, st));
-    CK(cudaMemsetAsync(scratch + kNoAllocDoneOff, 0, 4, st));
-    CK(cudaMemsetAsync(scratch + kNoAllocStatsOff, 0, (size_t)ST_COUNT * 8, st));
     p.cols = columns;
     p.S = n_samples;
     for (int k = 0; k < p.ncols; ++k) p.col_off[k] = (int64_t)p.vars[k] * pitch;
@@ -2755,6 +2775,9 @@ extern "C" int fpgm_ci_test_noalloc(const uint8_t *columns, int64_t pitch, int32
     p.stats = reinterpret_cast<unsigned long long *>(scratch + kNoAllocStatsOff);
     const int64_t nvec = n_samples >> 4;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(nvec / kThreads, 2 * nd->num_sms));
+    // the scratch keeps the previous call's contents: clear what must start at zero (a lone CTA
+    // keeps a table that fits its shared memory there)
+    if (grid > 1 || need > (double)kCtaInts) CK(cudaMemsetAsync(scratch, 0, (size_t)need * 4, st));
     ci_plain_kernel<<<grid, kThreads, kSmemBytes, st>>>(p);
     CK(cudaGetLastError());
     return FPGM_OK;
