@@ -2369,75 +2369,122 @@ struct MleNode {
     int32_t smem;   // 1: the table fits in shared memory
 };
 
-// One CTA per (node, slice of its samples): every sample's configuration code (Horner,
-// node first) counted in a shared-memory copy of the table when it fits, else in global
-// memory directly; 16 samples per thread step from 128-bit column loads.
-__global__ void __launch_bounds__(kThreads) mle_count_kernel(const uint8_t *cols, const int64_t *var_off,
-                                                             const int32_t *var_S, const uint8_t *card,
-                                                             const MleNode *nodes, const int32_t *parents,
-                                                             int32_t *counts) {
+// Least ints of shared memory per CTA: 40 KB, five CTAs to an SM; more where a table needs it.
+constexpr int kMleInts = 10240;
+// Entries up to which a node's last CTA forms its potentials; one SM divides for 30 us at 12,500.
+constexpr int kMleInline = 1024;
+constexpr int kMleLargeCtas = 32;  // CTAs of a larger table, at most
+
+// potential[j] = (N[j] + alpha) / (N(B of j) + alpha * card[v]), the reference's expression
+// (ParameterLearning.cpp:73-83) in FP64; N(B) sums the node's states for j's parent configuration.
+// The threads t, t + step, ... take an entry each where there are too few configurations for
+// all of them, else a configuration each, whose counts are added up once for all the node's states.
+__device__ inline void mle_potentials(const int32_t *tab, int cum0, int dv, int alpha, double *pot, int t, int step) {
+    if (cum0 < step) {
+        for (int64_t j = t; j < (int64_t)cum0 * dv; j += step) {
+            const int b = (int)((uint32_t)j % (uint32_t)cum0);  // a table has at most 2^30 entries
+            int sum = 0;
+            for (int a = 0; a < dv; ++a) sum += tab[(int64_t)a * cum0 + b];
+            pot[j] = ((double)tab[j] + alpha) / ((double)sum + alpha * dv);
+        }
+        return;
+    }
+    for (int64_t b = t; b < cum0; b += step) {
+        int sum = 0;
+        for (int a = 0; a < dv; ++a) sum += tab[(int64_t)a * cum0 + b];
+        const double den = (double)sum + alpha * dv;
+        for (int a = 0; a < dv; ++a) {
+            const int64_t j = (int64_t)a * cum0 + b;
+            pot[j] = ((double)tab[j] + alpha) / den;
+        }
+    }
+}
+
+// One CTA per (node, slice of its samples): every sample's configuration code (Horner, node
+// first) counted in replicas of the table in shared memory when it fits there, else in global
+// memory; the last CTA of a node to finish forms the potentials of a table of up to kMleInline
+// entries, taken back into shared memory (larger ones: mle_large_kernel).  Bound by the latency
+// of the chain descriptor - columns - counts - division; a table of a few cells by its
+// shared-memory atomics, which the replicas spread over the banks.  100 nodes of 50,000 samples:
+// 75 us for the call with a launch each for counts (without replicas) and potentials (one CTA a
+// node), 58 us now.
+__global__ void __launch_bounds__(kThreads) mle_kernel(const uint8_t *cols, const int64_t *var_off,
+                                                       const int32_t *var_S, const uint8_t *card,
+                                                       const MleNode *nodes, const int32_t *parents, int room,
+                                                       int32_t *counts, int32_t *done, int alpha, double *pot) {
     extern __shared__ int smem[];
     __shared__ const uint8_t *s_col[kMaxCols];
     __shared__ uint32_t s_dim[kMaxCols];
-    const int v = blockIdx.x;
+    __shared__ int s_last;
+    const int v = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
     const MleNode nd = nodes[v];
     const int ncols = nd.np + 1;
-    const int64_t S = var_S[v];
-    if (threadIdx.x < ncols) {
-        const int var = threadIdx.x == 0 ? v : parents[nd.par0 + threadIdx.x - 1];
-        s_col[threadIdx.x] = cols + var_off[var];
-        s_dim[threadIdx.x] = card[var];
-    }
-    const int64_t size = (int64_t)nd.cum0 * card[v];
-    int32_t *tab = nd.smem ? smem : counts + nd.off;
-    if (nd.smem)
-        for (int64_t i = threadIdx.x; i < size; i += blockDim.x) smem[i] = 0;
-    __syncthreads();
-    const int64_t nvec = S >> 4;
+    const int64_t S = var_S[v], nvec = S >> 4;
     const int64_t per = (nvec + gridDim.y - 1) / gridDim.y;
     const int64_t v0 = min(nvec, per * blockIdx.y), v1 = min(nvec, v0 + per);
-    for (int64_t q = v0 + threadIdx.x; q < v1; q += blockDim.x) {
-        uint32_t code[16];
-#pragma unroll
-        for (int b = 0; b < 16; ++b) code[b] = 0;
-        for (int j = 0; j < ncols; ++j) {
-            const uint4 w = __ldg(reinterpret_cast<const uint4 *>(s_col[j]) + q);
-            const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-            const uint32_t dm = s_dim[j];
-#pragma unroll
-            for (int b = 0; b < 16; ++b) code[b] = code[b] * dm + ((ww[b >> 2] >> (8 * (b & 3))) & 0xffu);
-        }
-#pragma unroll
-        for (int b = 0; b < 16; ++b) atomicAdd(&tab[code[b]], 1);
+    const int64_t n = (blockIdx.y == gridDim.y - 1 ? S : v1 * 16) - v0 * 16;  // the last slice has the ragged tail
+    if (tid < ncols) {
+        const int var = tid == 0 ? v : parents[nd.par0 + tid - 1];
+        s_col[tid] = cols + var_off[var] + v0 * 16;
+        s_dim[tid] = card[var];
     }
-    if (blockIdx.y == gridDim.y - 1)  // the ragged tail
-        for (int64_t s = (S & ~(int64_t)15) + threadIdx.x; s < S; s += blockDim.x) {
+    __syncthreads();
+    const int dv = s_dim[0];
+    const int64_t size = (int64_t)nd.cum0 * dv;
+    int32_t *tab = counts + nd.off;
+    if (nd.smem) {
+        int lgR = 0;
+        while (lgR < 5 && (size << (lgR + 1)) <= room && (size << (lgR + 3)) <= n) ++lgR;
+        const int R = 1 << lgR;
+        for (int i = tid; i < ((int)size << lgR); i += kThreads) smem[i] = 0;
+        __syncthreads();
+        count_columns(smem, lgR, lane, s_col, s_dim, ncols, n, tid, kThreads);
+        __syncthreads();
+        for (int c = tid; c < (int)size; c += kThreads) {
+            int m = 0;
+            for (int r = 0; r < R; ++r) m += smem[(c << lgR) + ((r + tid) & (R - 1))];
+            if (m) atomicAdd(&tab[c], m);
+        }
+    } else {
+        for (int64_t q = tid; q < n >> 4; q += kThreads) {
+            uint32_t code[16];
+#pragma unroll
+            for (int b = 0; b < 16; ++b) code[b] = 0;
+            for (int j = 0; j < ncols; ++j) {
+                const uint4 w = __ldg(reinterpret_cast<const uint4 *>(s_col[j]) + q);
+                const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+                const uint32_t dm = s_dim[j];
+#pragma unroll
+                for (int b = 0; b < 16; ++b) code[b] = code[b] * dm + ((ww[b >> 2] >> (8 * (b & 3))) & 0xffu);
+            }
+#pragma unroll
+            for (int b = 0; b < 16; ++b) atomicAdd(&tab[code[b]], 1);
+        }
+        for (int64_t s = (n & ~(int64_t)15) + tid; s < n; s += kThreads) {
             uint32_t c = 0;
             for (int j = 0; j < ncols; ++j) c = c * s_dim[j] + s_col[j][s];
             atomicAdd(&tab[c], 1);
         }
-    if (nd.smem) {
-        __syncthreads();
-        for (int64_t i = threadIdx.x; i < size; i += blockDim.x)
-            if (smem[i]) atomicAdd(&counts[nd.off + i], smem[i]);
     }
+    if (size > kMleInline) return;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(&done[v], 1) == (int)gridDim.y - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int i = tid; i < (int)size; i += kThreads) smem[i] = __ldcg(tab + i);
+    __syncthreads();
+    mle_potentials(smem, nd.cum0, dv, alpha, pot + nd.off, tid, kThreads);
 }
 
-// potential[j] = (N[j] + alpha) / (N(B of j) + alpha * card[v]), the reference's expression
-// (ParameterLearning.cpp:73-83) in FP64; N(B) sums the node's states for j's parent configuration.
-__global__ void mle_prob_kernel(const uint8_t *card, const MleNode *nodes, const int32_t *counts, int alpha,
-                                double *pot) {
-    const int v = blockIdx.x;
+// The potentials of the larger tables, several CTAs each: bound by the FP64 division.
+__global__ void __launch_bounds__(kThreads) mle_large_kernel(const uint8_t *card, const MleNode *nodes, const int32_t *large,
+                                                             const int32_t *counts, int alpha, double *pot) {
+    const int v = large[blockIdx.x];
     const MleNode nd = nodes[v];
-    const int dv = card[v];
-    const int64_t size = (int64_t)nd.cum0 * dv;
-    for (int64_t j = threadIdx.x; j < size; j += blockDim.x) {
-        const int64_t b = j % nd.cum0;
-        int num2 = 0;
-        for (int a = 0; a < dv; ++a) num2 += counts[nd.off + (int64_t)a * nd.cum0 + b];
-        const int num1 = counts[nd.off + j];
-        pot[nd.off + j] = ((double)num1 + alpha) / ((double)num2 + alpha * dv);
-    }
+    mle_potentials(counts + nd.off, nd.cum0, card[v], alpha, pot + nd.off, blockIdx.y * kThreads + threadIdx.x,
+                   gridDim.y * kThreads);
 }
 }  // namespace
 
@@ -2450,6 +2497,9 @@ extern "C" int fpgm_mle_cpts(fpgm_engine *e, const int32_t *parent_off, const in
     if (parent_off[0] != 0) return set_error(FPGM_ERR_INVALID, "fpgm_mle_cpts: parent_off[0] must be 0");
     std::vector<MleNode> nodes(n);
     int64_t total = 0;
+    int widest = 0;        // entries of the largest table counted in shared memory
+    int64_t largest = 0;   // of all
+    std::vector<int32_t> large;
     table_off[0] = 0;
     for (int v = 0; v < n; ++v) {
         const int np = parent_off[v + 1] - parent_off[v];
@@ -2474,35 +2524,48 @@ extern "C" int fpgm_mle_cpts(fpgm_engine *e, const int32_t *parent_off, const in
         nodes[v].np = np;
         nodes[v].par0 = parent_off[v];
         nodes[v].cum0 = (int32_t)cum0;
-        nodes[v].smem = size <= (double)(kSmemBytes / 4);
+        nodes[v].smem = size <= (double)kCtaInts;
+        if (nodes[v].smem) widest = std::max(widest, (int)size);
+        if (size > (double)kMleInline) large.push_back(v);
+        largest = std::max(largest, (int64_t)size);
         total += (int64_t)size;
         table_off[v + 1] = total;
     }
     if (!potentials) return FPGM_OK;
     CK(cudaSetDevice(e->device));
     const int64_t npar = std::max<int64_t>(parent_off[n], 1);
-    RET(e->mle_meta.ensure(sizeof(MleNode) * n + npar * 4 + 64));
-    RET(e->mle_counts.ensure((size_t)total * 4 + 16));
+    // [nodes | parent lists | large nodes], then [tables | CTAs done per node], cleared together
+    const size_t par_at = (sizeof(MleNode) * n + 15) / 16 * 16;
+    const size_t large_at = par_at + npar * 4;
+    std::vector<char> meta(large_at + large.size() * 4);
+    memcpy(meta.data(), nodes.data(), sizeof(MleNode) * n);
+    if (parent_off[n] > 0) memcpy(meta.data() + par_at, parents, (size_t)parent_off[n] * 4);
+    if (!large.empty()) memcpy(meta.data() + large_at, large.data(), large.size() * 4);
+    RET(e->mle_meta.ensure(meta.size()));
+    RET(e->mle_counts.ensure((size_t)(total + n) * 4));
     RET(e->mle_pot.ensure((size_t)total * 8 + 16));
-    MleNode *d_nodes = e->mle_meta.as<MleNode>();
-    int32_t *d_par = reinterpret_cast<int32_t *>(e->mle_meta.as<char>() + (sizeof(MleNode) * n + 15) / 16 * 16);
-    CK(cudaMemcpyAsync(d_nodes, nodes.data(), sizeof(MleNode) * n, cudaMemcpyHostToDevice, e->stream));
-    if (parent_off[n] > 0)
-        CK(cudaMemcpyAsync(d_par, parents, (size_t)parent_off[n] * 4, cudaMemcpyHostToDevice, e->stream));
-    CK(cudaMemsetAsync(e->mle_counts.p, 0, (size_t)total * 4, e->stream));
+    CK(cudaMemcpyAsync(e->mle_meta.p, meta.data(), meta.size(), cudaMemcpyHostToDevice, e->stream));
+    CK(cudaMemsetAsync(e->mle_counts.p, 0, (size_t)(total + n) * 4, e->stream));
     // slices per node: enough CTAs to fill the GPU, at least 64 vectors each
     int64_t smax = 0;
     for (int v = 0; v < n; ++v) smax = std::max<int64_t>(smax, e->h_var_S[v]);
     const int want = std::max(1, (4 * e->num_sms + n - 1) / n);
     const int slices = (int)std::max<int64_t>(1, std::min<int64_t>(want, (smax >> 4) / 64));
-    CK(cudaFuncSetAttribute(mle_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    mle_count_kernel<<<dim3(n, slices), kThreads, kSmemBytes, e->stream>>>(
-        e->cols.as<uint8_t>(), e->var_off.as<int64_t>(), e->var_S.as<int32_t>(), e->card.as<uint8_t>(), d_nodes, d_par,
-        e->mle_counts.as<int32_t>());
+    const int room = std::max(kMleInts, (widest + 1023) / 1024 * 1024);
+    if (room > kMleInts) CK(cudaFuncSetAttribute(mle_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    mle_kernel<<<dim3(n, slices), kThreads, (size_t)room * 4, e->stream>>>(
+        e->cols.as<uint8_t>(), e->var_off.as<int64_t>(), e->var_S.as<int32_t>(), e->card.as<uint8_t>(),
+        e->mle_meta.as<MleNode>(), reinterpret_cast<const int32_t *>(e->mle_meta.as<char>() + par_at), room,
+        e->mle_counts.as<int32_t>(), e->mle_counts.as<int32_t>() + total, alpha, e->mle_pot.as<double>());
     CK(cudaGetLastError());
-    mle_prob_kernel<<<n, kThreads, 0, e->stream>>>(e->card.as<uint8_t>(), d_nodes, e->mle_counts.as<int32_t>(), alpha,
-                                                  e->mle_pot.as<double>());
-    CK(cudaGetLastError());
+    if (!large.empty()) {
+        const int ctas = (int)std::min<int64_t>(kMleLargeCtas, (largest + kThreads - 1) / kThreads);
+        mle_large_kernel<<<dim3((unsigned)large.size(), ctas), kThreads, 0, e->stream>>>(
+            e->card.as<uint8_t>(), e->mle_meta.as<MleNode>(),
+            reinterpret_cast<const int32_t *>(e->mle_meta.as<char>() + large_at), e->mle_counts.as<int32_t>(), alpha,
+            e->mle_pot.as<double>());
+        CK(cudaGetLastError());
+    }
     CK(cudaMemcpyAsync(potentials, e->mle_pot.p, (size_t)total * 8, cudaMemcpyDeviceToHost, e->stream));
     CK(cudaStreamSynchronize(e->stream));
     return FPGM_OK;

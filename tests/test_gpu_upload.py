@@ -20,6 +20,20 @@ def eng():
     e.close()
 
 
+@pytest.mark.parametrize("S", [1, 15, 1025, 2048 * 16 + 3, 100007])
+@pytest.mark.parametrize("card", [(2, 2), (3, 9)])
+def test_parameter_tables(eng, S, card):
+    """0 to 5 parents: one slice and several, byte and 16-bit codes, one and many replicas, tables
+    of one entry per thread and of more configurations than threads."""
+    raw, _, par = F.generate(n_nodes=12, n_samples=S, seed=5, n_edges=26, max_indegree=5, card=card)
+    cols, states = O.relabel(raw)
+    eng.upload(raw)
+    parents = [par[v] for v in range(raw.shape[0])]
+    got = eng.mle_cpts(parents, alpha=1)
+    for v, (g, o) in enumerate(zip(got, O.mle_cpts(cols, states, parents, alpha=1))):
+        assert g.shape == o.shape and np.array_equal(g, o), v
+
+
 @pytest.mark.parametrize("S", [1, 15, 16, 4096, 8192, 40007])
 def test_single_tests(eng, S):
     """fpgm_ci_test and its allocation-free form on one CTA and on several: counts, df and
