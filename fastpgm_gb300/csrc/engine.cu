@@ -248,46 +248,91 @@ struct fpgm_engine {
 namespace {
 
 // ---- data preparation
-// First-appearance ids per column (Dataset.cpp:459-467) and observed cardinality.
-__global__ void relabel_kernel(uint8_t *cols, const int64_t *var_off, const int32_t *var_S, uint8_t *card,
-                               int relabel) {
-    __shared__ unsigned first[256];
+// First-appearance ids per column (Dataset.cpp:459-467) and observed cardinality: a cluster of
+// kSlices CTAs per column.  Every thread looks for the first place of each value among its own
+// samples, 16 a load: which of the values below 32 it has met is a mask in a register, so that
+// almost all of the samples cost no access to shared memory.  The cluster's first places meet in
+// its first CTA, a value's id is the number of values that appear before it, and each CTA maps
+// its own samples.  Bound by the latency of its passes at 5,000 samples (37 columns: 7 us, 31 us
+// with one CTA per column and single bytes) and 50,000 (100 columns: 16 us, was 95 us), by
+// instruction issue at 500,000 (223 columns: 84 us, was 839 us).
+constexpr int kRelabelThreads = 512;
+// Samples from which a column is worth a cluster: below, one CTA has it in two loads a thread.
+constexpr int64_t kRelabelSliced = 16384;
+template <int kSlices>
+__global__ void __cluster_dims__(kSlices, 1, 1) __launch_bounds__(kRelabelThreads)
+    relabel_kernel(uint8_t *cols, const int64_t *var_off, const int32_t *var_S, uint8_t *card, int relabel) {
+    __shared__ unsigned first[256], all[256];
     __shared__ uint8_t map[256];
-    __shared__ unsigned s_max;
-    uint8_t *c = cols + var_off[blockIdx.x];
-    const int64_t S = var_S[blockIdx.x];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) first[i] = 0xffffffffu;
-    if (threadIdx.x == 0) s_max = 0;
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int col = blockIdx.x / kSlices, slice = blockIdx.x % kSlices, tid = threadIdx.x;
+    uint8_t *c = cols + var_off[col];
+    uint4 *cv = reinterpret_cast<uint4 *>(c);
+    const unsigned S = (unsigned)var_S[col], nvec = S >> 4;
+    const unsigned per = (nvec + kSlices - 1) / kSlices, v0 = min(nvec, per * slice), v1 = min(nvec, v0 + per);
+    const unsigned tail = slice == kSlices - 1 ? nvec * 16 : S;  // the last slice has the ragged end
+    if (tid < 256) first[tid] = 0xffffffffu;
     __syncthreads();
-    if (relabel) {
-        for (int64_t s = threadIdx.x; s < S; s += blockDim.x) {
-            unsigned v = c[s];
-            if ((unsigned)s < first[v]) atomicMin(&first[v], (unsigned)s);
+    uint32_t seen = 0;
+    auto look = [&](unsigned v, unsigned s) {
+        if (v < 32) {
+            if (seen >> v & 1u) return;
+            seen |= 1u << v;
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int next = 0;
-            // values sorted by first appearance: repeated min-selection over <= 256 values
-            bool used[256];
-            for (int i = 0; i < 256; ++i) used[i] = first[i] == 0xffffffffu;
-            for (;;) {
-                int best = -1;
-                unsigned bp = 0xffffffffu;
-                for (int i = 0; i < 256; ++i)
-                    if (!used[i] && first[i] < bp) { bp = first[i]; best = i; }
-                if (best < 0) break;
-                used[best] = true;
-                map[best] = (uint8_t)next++;
-            }
-            card[blockIdx.x] = (uint8_t)next;
-        }
-        __syncthreads();
-        for (int64_t s = threadIdx.x; s < S; s += blockDim.x) c[s] = map[c[s]];
-    } else {
-        for (int64_t s = threadIdx.x; s < S; s += blockDim.x) atomicMax(&s_max, (unsigned)c[s]);
-        __syncthreads();
-        if (threadIdx.x == 0) card[blockIdx.x] = (uint8_t)(s_max + 1);
+        if (s < first[v]) atomicMin(&first[v], s);
+    };
+    unsigned q = v0 + tid;
+    uint4 w = q < v1 ? cv[q] : make_uint4(0, 0, 0, 0);
+    for (; q < v1; q += kRelabelThreads) {
+        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+        if (q + kRelabelThreads < v1) w = cv[q + kRelabelThreads];
+        bool any = ((ww[0] | ww[1] | ww[2] | ww[3]) & 0xe0e0e0e0u) != 0;
+        uint32_t m = 0;
+#pragma unroll
+        for (int b = 0; b < 16; ++b) m |= 1u << ((ww[b >> 2] >> (8 * (b & 3))) & 31u);
+        if (any || (m & ~seen))
+            for (int b = 0; b < 16; ++b) look((ww[b >> 2] >> (8 * (b & 3))) & 0xffu, q * 16 + b);
     }
+    for (unsigned s = tail + tid; s < S; s += kRelabelThreads) look(c[s], s);
+    __syncthreads();
+    if (kSlices > 1) {
+        cluster.sync();
+        if (slice != 0 && tid < 256 && first[tid] != 0xffffffffu)
+            atomicMin(cluster.map_shared_rank(&first[tid], 0), first[tid]);
+        cluster.sync();
+        if (tid < 256) all[tid] = *cluster.map_shared_rank(&first[tid], 0);
+        cluster.sync();
+    } else if (tid < 256) {
+        all[tid] = first[tid];
+    }
+    const bool used = tid < 256 && all[tid & 255] != 0xffffffffu;
+    const int states = __syncthreads_count(used);
+    if (!relabel) {  // values as given: the largest + 1 (256 wraps to 0)
+        if (slice == 0 && used) {
+            bool top = true;
+            for (int v = tid + 1; v < 256; ++v) top = top && all[v] == 0xffffffffu;
+            if (top) card[col] = (uint8_t)(tid + 1);
+        }
+        return;
+    }
+    if (used) {
+        int id = 0;
+        for (int v = 0; v < 256; ++v) id += all[v] < all[tid];
+        map[tid] = (uint8_t)id;
+    }
+    if (slice == 0 && tid == 0) card[col] = (uint8_t)states;
+    __syncthreads();
+    for (unsigned p = v0 + tid; p < v1; p += kRelabelThreads) {
+        const uint4 u = cv[p];
+        const uint32_t uu[4] = {u.x, u.y, u.z, u.w};
+        uint32_t o[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            o[k] = (uint32_t)map[uu[k] & 0xffu] | (uint32_t)map[(uu[k] >> 8) & 0xffu] << 8 |
+                   (uint32_t)map[(uu[k] >> 16) & 0xffu] << 16 | (uint32_t)map[uu[k] >> 24] << 24;
+        cv[p] = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+    for (unsigned s = tail + tid; s < S; s += kRelabelThreads) c[s] = map[c[s]];
 }
 
 // ---- level machinery
@@ -1072,8 +1117,12 @@ int load_datasets(fpgm_engine *e, int32_t n_jobs, const int32_t *job_vars, const
     CK(cudaMemcpyAsync(e->var_S.p, e->h_var_S.data(), (size_t)n * 4, cudaMemcpyHostToDevice, e->stream));
     CK(cudaMemcpyAsync(e->var_lo.p, e->h_var_lo.data(), (size_t)n * 4, cudaMemcpyHostToDevice, e->stream));
     CK(cudaMemcpyAsync(e->var_hi.p, e->h_var_hi.data(), (size_t)n * 4, cudaMemcpyHostToDevice, e->stream));
-    relabel_kernel<<<(int)n, 256, 0, e->stream>>>(e->cols.as<uint8_t>(), e->var_off.as<int64_t>(),
-                                                  e->var_S.as<int32_t>(), e->card.as<uint8_t>(), relabel);
+    if (smax >= kRelabelSliced)
+        relabel_kernel<8><<<(int)n * 8, kRelabelThreads, 0, e->stream>>>(
+            e->cols.as<uint8_t>(), e->var_off.as<int64_t>(), e->var_S.as<int32_t>(), e->card.as<uint8_t>(), relabel);
+    else
+        relabel_kernel<1><<<(int)n, kRelabelThreads, 0, e->stream>>>(
+            e->cols.as<uint8_t>(), e->var_off.as<int64_t>(), e->var_S.as<int32_t>(), e->card.as<uint8_t>(), relabel);
     CK(cudaGetLastError());
     e->h_card.resize(n);
     CK(cudaMemcpyAsync(e->h_card.data(), e->card.p, n, cudaMemcpyDeviceToHost, e->stream));

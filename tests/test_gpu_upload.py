@@ -20,6 +20,49 @@ def eng():
     e.close()
 
 
+def _columns(S, seed):
+    """Columns of 1, 2, 31, 33 and 255 states (as far as S allows), a constant one, one whose only
+    other value is the last sample, and one in descending order of first appearance."""
+    rng = np.random.default_rng(seed)
+    cols = [rng.integers(0, k, size=S) for k in (2, 31, 33, 255)]
+    cols.append(np.full(S, 200))
+    late = np.full(S, 7)
+    late[-1] = 3
+    cols.append(late)
+    cols.append(np.maximum(0, 40 - np.arange(S)))
+    return np.stack(cols).astype(np.uint8)
+
+
+@pytest.mark.parametrize("S", [1, 15, 16, 17, 8191, 16383, 16384, 16385, 65536 + 5, 200003])
+def test_relabel(eng, S):
+    raw = _columns(S, S)
+    want = np.empty_like(raw)
+    states = []
+    for v, c in enumerate(raw):
+        _, first, inv = np.unique(c, return_index=True, return_inverse=True)
+        rank = np.empty(len(first), dtype=np.uint8)
+        rank[np.argsort(first)] = np.arange(len(first), dtype=np.uint8)
+        want[v] = rank[inv]
+        states.append(len(first))
+    card = eng.upload(raw)
+    assert np.array_equal(card, states)
+    assert np.array_equal(eng.download(), want)
+    # as given: the values stay and the cardinality is the largest + 1
+    card = eng.upload(raw, relabel=False)
+    assert np.array_equal(card, raw.max(axis=1).astype(int) + 1)
+    assert np.array_equal(eng.download(), raw)
+
+
+@pytest.mark.parametrize("S", [300, 40000])
+def test_256_states_are_refused(eng, S):
+    raw = np.zeros((3, S), dtype=np.uint8)
+    raw[1] = np.arange(S) % 256
+    with pytest.raises(F.FpgmError):
+        eng.upload(raw)
+    with pytest.raises(F.FpgmError):
+        eng.upload(raw, relabel=False)
+
+
 @pytest.mark.parametrize("S", [1, 15, 1025, 2048 * 16 + 3, 100007])
 @pytest.mark.parametrize("card", [(2, 2), (3, 9)])
 def test_parameter_tables(eng, S, card):
