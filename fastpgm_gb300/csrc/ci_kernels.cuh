@@ -138,6 +138,15 @@ struct SetArgs {
     int32_t few;               // at most this many new sets: each is counted by a whole CTA
 };
 
+// G^2 of a pair of three variables given the third: entry at of the sets of three (SetArgs::key)
+// has it at g[3 at + c], given the c-th of its variables in ascending order; NaN: not known.
+struct TripleArgs {
+    const uint64_t *key;  // null: not kept
+    int32_t cap, probe;
+    float *g;
+    int32_t *listed;      // per entry, while they are computed
+};
+
 struct WaveArgs {
     const uint8_t *cols;
     const int64_t *var_off;  // byte offset of each variable's column in cols
@@ -176,6 +185,7 @@ struct WaveArgs {
     int32_t n_vars;
     Fixed fx;              // fixed-point statistic of tests that need no detail
     SetArgs sets;
+    TripleArgs tri;        // of level 2's edges and neighbours (sets.cuh)
     int32_t strata_card;   // tests whose other endpoint has at most this many states go to list 6 (0: none)
     // compact tier: per-CTA global slots
     char *slot_mem;
@@ -341,12 +351,15 @@ __host__ __device__ inline int set_class(int cells, int64_t S) {
     return k;
 }
 
+// Key of a set of two (w = 0xffff) or three ascending variables, or of the first three of more.
+__device__ inline uint64_t set_key(int u, int v, int w) {
+    return (1ull << 62) | (uint64_t)u << 32 | (uint64_t)v << 16 | (uint64_t)w;
+}
 // Entry of the set of m >= 2 ascending variables: the first three in one key, then two at a
 // time after the entry reached so far (the keys hold the variables themselves, so two sets
 // never share an entry).  -1: no room.
 __device__ inline int set_enter(const SetArgs &s, const uint16_t *v, int m, bool *fresh) {
-    int at = table_enter(s.key, s.cap, s.probe, (1ull << 62) | (uint64_t)v[0] << 32 | (uint64_t)v[1] << 16 | (m > 2 ? v[2] : 0xffffu),
-                         fresh);
+    int at = table_enter(s.key, s.cap, s.probe, set_key(v[0], v[1], m > 2 ? v[2] : 0xffff), fresh);
     for (int i = 3; i < m && at >= 0; i += 2)
         at = table_enter(s.key, s.cap, s.probe,
                          (1ull << 63) | (uint64_t)at << 32 | (uint64_t)v[i] << 16 | (i + 1 < m ? v[i + 1] : 0xffffu), fresh);
@@ -378,6 +391,35 @@ __device__ inline bool dependent_by_pairs(const WaveArgs &a, int x, int y, int z
 __device__ inline void keep_pair(const WaveArgs &a, int x, int y, double g2) {
     a.pair_g2[(int64_t)x * a.n_vars + y] = (float)g2;
     a.pair_g2[(int64_t)y * a.n_vars + x] = (float)g2;
+}
+
+// G^2(a, b | c), NaN when it was not kept.
+__device__ inline float triple_g2(const TripleArgs &t, int a, int b, int c) {
+    const int lo = min(a, b), hi = max(a, b);
+    const int u = min(lo, c), w = max(hi, c), v = lo + hi + c - u - w;
+    const uint64_t key = set_key(u, v, w);
+    uint32_t h = (uint32_t)((key * 0x9E3779B97F4A7C15ull) >> 32) & (uint32_t)(t.cap - 1);
+    for (int p = 0; p < t.probe; ++p) {
+        const uint64_t k = __ldg(t.key + h);
+        if (k == key) return __ldg(t.g + 3 * (int64_t)h + (c == u ? 0 : (c == v ? 1 : 2)));
+        if (k == 0) break;
+        h = (h + 1) & (uint32_t)(t.cap - 1);
+    }
+    return __int_as_float(0x7fffffff);
+}
+// The chain rule at level 2: I(x; y | z w) = I(x; y | z) + I(x; w | y z) - I(x; w | z) is at least
+// I(x; y | z) - min(I(x; w | z), I(y; w | z)), for either order of Z.
+__device__ inline bool dependent_by_triples(const WaveArgs &a, int x, int y, int z0, int z1, int64_t df) {
+    if (df > a.fx.dfmax) return false;
+    const float hi = (float)a.fx.hi[df] * 1.000001f;
+    for (int k = 0; k < 2; ++k) {
+        const int z = k ? z1 : z0, w = k ? z0 : z1;
+        const float xy = triple_g2(a.tri, x, y, z);
+        if (!(xy > hi)) continue;
+        const float off = fminf(triple_g2(a.tri, x, w, z), triple_g2(a.tri, y, w, z));  // the known one of two
+        if (xy - off - 1e-6f * (xy + off) - 1e-3f > hi) return true;
+    }
+    return false;
 }
 
 // Item -> (x, y, Z) -> tier.  One thread per item, grid-stride.
@@ -419,7 +461,10 @@ __global__ void classify_kernel(WaveArgs a) {
             const bool known =
                 (side == 1 && a.bits && tested_from_x(a, x, z)) ||
                 (d == 1 && a.pair_g2 &&
-                 dependent_by_pairs(a, x, y, z[0], (int64_t)(a.card[x] - 1) * (a.card[y] - 1) * a.card[z[0]]));
+                 dependent_by_pairs(a, x, y, z[0], (int64_t)(a.card[x] - 1) * (a.card[y] - 1) * a.card[z[0]])) ||
+                (d == 2 && a.tri.key &&
+                 dependent_by_triples(a, x, y, z[0], z[1],
+                                      (int64_t)(a.card[x] - 1) * (a.card[y] - 1) * a.card[z[0]] * a.card[z[1]]));
             if (known) {
                 a.flag[item] = 0;
                 continue;

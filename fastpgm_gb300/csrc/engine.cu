@@ -235,7 +235,10 @@ struct fpgm_engine {
     size_t set_pool_fixed = 0, strata_pool_fixed = 0;  // FPGM_SET_POOL, FPGM_STRATA_POOL (tests): bytes
     DevBuf set_tab, set_pool, set_items;
     DevBuf pair_g2;                     // level 0's statistics, read at level 1 (FPGM_BOUND=0: not kept)
-    bool bound_on = true, pairs_kept = false;
+    bool bound_on = true, pairs_kept = false, bound_all = false;  // (FPGM_BOUND=2: whatever the size)
+    DevBuf tri_tab, tri_g;              // level 1's set table, kept for level 2, and its statistics
+    int32_t tri_cap = 0, tri_probe = 0;
+    bool tri_ready = false;
     bool tune_loaded = false, tune_online = true;
     std::string tune_source;
     // result
@@ -966,6 +969,7 @@ extern "C" int fpgm_engine_create(int32_t device, fpgm_engine **out) {
                             kWarps * kWarpIntsSmall * 4));
     CK(cudaFuncSetAttribute(set_count_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     CK(cudaFuncSetAttribute(set_score_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    CK(cudaFuncSetAttribute(triple_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWarps * kTripleInts * 4));
     CK(cudaFuncSetAttribute(strata_test_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTestInts * 4));
     CK(cudaFuncSetAttribute(ci_plain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
     int occ = 0;
@@ -1000,7 +1004,7 @@ extern "C" int fpgm_engine_create(int32_t device, fpgm_engine **out) {
     if (const char *w = getenv("FPGM_GRAPH")) e->graph_on = atoi(w) != 0;
     if (const char *w = getenv("FPGM_STRATA")) e->strata_on = atoi(w) != 0;
     if (const char *w = getenv("FPGM_SETS")) e->sets_on = atoi(w) != 0;
-    if (const char *w = getenv("FPGM_BOUND")) e->bound_on = atoi(w) != 0;
+    if (const char *w = getenv("FPGM_BOUND")) e->bound_on = atoi(w) != 0, e->bound_all = atoi(w) > 1;
     if (const char *w = getenv("FPGM_SET_POOL")) e->set_pool_fixed = (size_t)std::max(16ll, atoll(w));
     if (const char *w = getenv("FPGM_STRATA_POOL")) e->strata_pool_fixed = (size_t)std::max(16ll, atoll(w));
     e->gram = gram_create();
@@ -1048,7 +1052,7 @@ extern "C" int fpgm_engine_destroy(fpgm_engine *e) {
                       &e->tune_obs, &e->ovf, &e->live_pool[0], &e->live_pool[1], &e->live_tab[0], &e->live_tab[1],
                       &e->live_cnt, &e->live_stat, &e->res_adj_d, &e->res_key, &e->res_idx, &e->res_removed_d, &e->res_cnt,
                       &e->res_vars_d, &e->fixed_f, &e->tight, &e->set_tab,
-                      &e->set_pool, &e->set_items, &e->pair_g2, &e->strata_tab, &e->strata_lists, &e->strata_pool,
+                      &e->set_pool, &e->set_items, &e->pair_g2, &e->tri_tab, &e->tri_g, &e->strata_tab, &e->strata_lists, &e->strata_pool,
                       &e->strata_refs, &e->strata_used};
     for (DevBuf *b : bufs) b->release();
     gram_destroy(e->gram);
@@ -1526,6 +1530,12 @@ int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t ite
         a.bit_words = (e->n + 31) / 32;
         a.n_vars = e->n;
         if (a.fx.f && d <= 1 && e->pairs_kept) a.pair_g2 = e->pair_g2.as<float>();
+        if (a.fx.f && d == 2 && e->tri_ready) {
+            a.tri.key = reinterpret_cast<uint64_t *>(e->tri_tab.as<char>() + 16);
+            a.tri.cap = e->tri_cap;
+            a.tri.probe = e->tri_probe;
+            a.tri.g = e->tri_g.as<float>();
+        }
     }
     if (e->sets_level) {
         const size_t ni = (size_t)std::max<int64_t>(items, 1);
@@ -1550,6 +1560,50 @@ int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t ite
     a.warp_ints = e->warp_small ? kWarpIntsSmall : kWarpInts;
     a.dense_rows = e->dense_rows;
     a.stage_rec = e->stage_rec;
+    return FPGM_OK;
+}
+
+// Level 2's bounds (triple_enter_kernel), before its waves and before its own set table takes
+// the place of level 1's.  Off where level 1 kept no sets; and below kTripleWork samples of tests
+// (their bound times the samples), where the launches cost more than they save: 61 variables x
+// 20,011 samples 0.20 ms without and 0.26 with, 37 x 5,000 0.084 and 0.141; equal (0.78 ms) for
+// 60,000 tests of eight datasets of up to 40,000 samples.
+constexpr double kTripleWork = 3e9;
+int triples_setup(fpgm_engine *e, double alpha, const WaveArgs &proto, int64_t n_active, int64_t max_deg,
+                  fpgm_pc_stats *st) {
+    e->tri_ready = false;
+    if (!e->bound_on || !e->sets_level || !e->in_skeleton || e->fixed_n < e->S ||
+        ((double)e->level_tests * (double)e->S < kTripleWork && !e->bound_all))
+        return FPGM_OK;
+    const int64_t items = std::min<int64_t>(2 * n_active * std::max<int64_t>(max_deg - 1, 1), 1 << 20);
+    const size_t g_bytes = (size_t)e->sets_cap * 12;
+    if (e->tri_g.ensure(g_bytes + (size_t)e->sets_cap * 4) != FPGM_OK) return FPGM_OK;
+    WaveArgs a;
+    RET(wave_args_base(e, a, alpha, 1, items));
+    a.adjl = proto.adjl;
+    a.adj_stride = proto.adj_stride;
+    a.deg = proto.deg;
+    a.ex = proto.ex;
+    a.ey = proto.ey;
+    a.pxy = proto.pxy;
+    a.pyx = proto.pyx;
+    a.n_edges = (int32_t)n_active;
+    a.tri.g = e->tri_g.as<float>();
+    a.tri.listed = reinterpret_cast<int32_t *>(e->tri_g.as<char>() + g_bytes);
+    CK(cudaMemsetAsync(a.tri.g, 0xff, g_bytes, e->stream));  // NaN
+    CK(cudaMemsetAsync(a.tri.listed, 0, (size_t)e->sets_cap * 4, e->stream));
+    CK(cudaMemsetAsync(e->counters.p, 0, kCounterBytes, e->stream));
+    triple_enter_kernel<<<blocks_for(n_active * 32, kThreads), kThreads, 0, e->stream>>>(a);
+    CK(cudaGetLastError());
+    set_count_kernel<<<3 * e->num_sms, kThreads, kWarps * kSetWarpInts * 4, e->stream>>>(a);
+    CK(cudaGetLastError());
+    triple_score_kernel<<<3 * e->num_sms, kThreads, kWarps * kTripleInts * 4, e->stream>>>(a);
+    CK(cudaGetLastError());
+    st->kernel_launches += 3;
+    std::swap(e->set_tab, e->tri_tab);
+    e->tri_cap = a.sets.cap;
+    e->tri_probe = a.sets.probe;
+    e->tri_ready = true;
     return FPGM_OK;
 }
 
@@ -2049,6 +2103,7 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
             double ranks = 2.0;
             for (int k = 0; k < d; ++k) ranks = std::min(1e15, ranks * std::max(0, max_deg - 1 - k) / (k + 1));
             e->level_tests = d == 0 ? n_active : (int64_t)std::min(1e15, ranks * (double)n_active) + 64;
+            if (d == 2) RET(triples_setup(e, alpha, a, n_active, max_deg, st));
             if (!gram) RET(sets_setup(e, d, n_active));
             if (d == 0 && !gram && !(e->sets_level && e->sets_all)) e->pairs_kept = false;  // some tests count their own
             RET(strata_setup(e, d, d <= 1, e->level_host->strata_used));

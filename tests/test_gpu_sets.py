@@ -90,3 +90,37 @@ def test_level_1_bounds_across_datasets():
         cols, card = O.relabel(raw)
         ref = O.pc_skeleton(cols, card, threads=16)
         assert np.array_equal(adj, ref["adj"]) and seps == ref["sepsets"]
+
+
+@pytest.mark.parametrize("pool", [None, "16", "20000"])
+@pytest.mark.parametrize("n,S,card,edges,alpha", [(40, 3000, (2, 3), 70, 0.05), (30, 20000, (2, 9), 45, 0.05),
+                                                  (25, 4000, (2, 4), 60, 0.0), (25, 4000, (2, 4), 60, 0.9),
+                                                  (20, 15, (2, 3), 40, 0.3), (16, 9000, (11, 15), 20, 1e-4)])
+def test_level_2_bounds_match_oracle(monkeypatch, pool, n, S, card, edges, alpha):
+    """Level 2 decided from its sets of three variables at sizes below the rule's (FPGM_BOUND=2);
+    sets whose tables found no room, or are past a warp's 2,048 cells, bound nothing."""
+    monkeypatch.setenv("FPGM_BOUND", "2")
+    if pool:
+        monkeypatch.setenv("FPGM_SET_POOL", pool)
+    raw, _, _ = F.generate(n_nodes=n, n_samples=S, seed=n + S, n_edges=edges, max_indegree=4, card=card)
+    rng = np.random.default_rng(n)
+    for v in range(0, n - 2, 4):  # noisy copies: dependence that one or two neighbours explain in part
+        for k in (1, 2):
+            keep = rng.random(S) < rng.uniform(0.05, 0.9)
+            raw[v + k, keep] = raw[v, keep]
+    _check(raw, depth=5, alpha=alpha)
+
+
+def test_level_2_bounds_across_datasets(monkeypatch):
+    monkeypatch.setenv("FPGM_BOUND", "2")
+    data = [F.generate(n_nodes=n, n_samples=S, seed=S, n_edges=2 * n, max_indegree=4, card=(2, 5))[0]
+            for n, S in ((12, 700), (30, 9000), (2, 40), (17, 2500))]
+    with F.Engine(0) as e:
+        for _ in range(2):  # the second pass finds the buffers of the first
+            e.upload_jobs(data)
+            e.pc_skeleton()
+            res = e.result()
+            for raw, (adj, seps) in zip(data, F.split_jobs(res, e.job_offsets)):
+                cols, card = O.relabel(raw)
+                ref = O.pc_skeleton(cols, card, threads=16)
+                assert np.array_equal(adj, ref["adj"]) and seps == ref["sepsets"]
