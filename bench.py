@@ -320,7 +320,7 @@ def kernel_groups(tot, config, peak, peak_kind):
     the larger share first."""
     kernels = []
     for name, desc, members, ms, nbytes in (
-            ("ci_warp_kernel", "classify + warp-per-test + CTA-per-test kernels, shared-memory tables",
+            ("ci_warp_kernel", "classify + tables shared by variable set (or a test's own), shared memory",
              ("ci_warp_kernel",), tot["count_ms"], tot["count_bytes"]),
             ("ci_compact_kernel+ci_part_kernel",
              "tier 2, joint tables beyond shared memory: hashed strata (compact kernel) and partitioned "

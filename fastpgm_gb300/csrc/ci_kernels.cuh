@@ -1,6 +1,10 @@
 // CI-test kernels of the engine.  Every test of a wave (or of an explicit
-// batch) is first classified by the size of its joint table and sent to one
-// of three persistent kernels:
+// batch) is first classified.  A skeleton's tests are decided without a count
+// where earlier ones imply the outcome (tested_from_x, dependent_by_pairs,
+// dependent_by_triples), else from tables shared by variable set (sets.cuh)
+// or from shared strata (strata.cuh).  An explicit batch's tests, and those
+// that find no room there, go by the size of their joint table to one of
+// three persistent kernels:
 //
 //   tier 0  ci_warp_kernel     one warp per test, table + marginals in a 12 KB
 //                              per-warp slice of shared memory (<= 3072 ints)

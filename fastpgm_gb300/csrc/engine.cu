@@ -8,8 +8,8 @@
 //     y-side sets, each in the lexicographic order of ChoiceGenerator
 //     (CheckEdge :399-494, ChoiceGenerator.cpp:55-85);
 //   * a level runs in waves; a wave gives each unresolved edge the next q
-//     ranks (q grows geometrically), one persistent kernel drains all tests
-//     of the wave from a work counter, and a reduction keeps, per edge, the
+//     ranks (q grows geometrically), persistent kernels drain the wave's sets
+//     and tests from work counters, and a reduction keeps, per edge, the
 //     FIRST independent rank -- the reference's sepset (Testing :526-614);
 //   * removals are applied to the bitset at the end of the level and the
 //     FreeDegree stop rule (:620-626, :387) is evaluated on the device.

@@ -268,9 +268,10 @@ __global__ void __launch_bounds__(kThreads, 2) set_score_cta_kernel(WaveArgs a) 
 // (dependent_by_triples), which are far fewer than its tests: of a variable of k neighbours
 // C(k, 2) against k C(k - 1, 2).  Before the level's first wave those of every edge and neighbour
 // are completed from level 1's tables, which hold most of them counted, and the rest is counted
-// now.  The bound decides 91% of level 2's tests with 100 variables x 50,000 samples, 97% with
-// 223 x 500,000 and 89% with 1,041 x 100,000 (sampled); the level takes 1.20, 7.96 and 13.3 ms
-// where it took 1.68, 17.7 and 23.7.
+// now.  It leaves 22% of the tests run at level 2 to be counted with 100 variables x 50,000
+// samples, 18% with 223 x 500,000 and 62% with 1,041 x 100,000 (tested_from_x included); the level
+// takes 1.20, 7.96 and 13.3 ms where it took 1.68, 17.7 and 23.7.  The sets {y, z, w} with z and w
+// neighbours of x alone would leave 3 to 11%, but they are as many as the sets of four.
 constexpr int kTripleInts = 2048;  // the largest table taken (a warp's shared memory)
 
 // One warp per edge of the level (a: level 1's sets; d = 1), a lane per neighbour of either end.

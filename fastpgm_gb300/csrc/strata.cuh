@@ -185,13 +185,13 @@ __device__ __forceinline__ long long block_sum_ll(long long v, long long *scratc
 // strata in the low halves (when 32-bit ones would not fit and no stratum of P has more samples
 // than 16 bits hold).
 struct StrataRows {
-    uint32_t r0, nr;    // strata counted in this round
+    uint32_t r0, nr;    // strata counted in this pass
     uint32_t split;     // strata of the round in low halves (wide: all)
     uint32_t cv, mul;   // values of v; bytes from one word's copy to the next word's
     uint32_t base;      // shared-memory address of this lane's copy
 };
 
-// Adds one sample (16 bits of id, a byte of v) when its stratum is of this round.
+// Adds one sample (16 bits of id, a byte of v) when its stratum is of this pass.
 __device__ __forceinline__ void strata_add(const StrataRows &g, uint32_t id, uint32_t value) {
     uint32_t k = id - g.r0;
     if (k >= g.nr) return;  // kNoStratum is past every round's last stratum (n <= 65,534)

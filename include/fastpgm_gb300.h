@@ -79,12 +79,13 @@ typedef struct {
     int32_t edges_after[64];     /* skeleton edges left after the level */
     int32_t waves[64];           /* batched waves in the level */
     double ms[64];               /* wall time of the level, host clock around device work */
-    int64_t rechecks;            /* tests that entered the FP64 band */
+    int64_t rechecks;            /* tests that neither the FP32 bound nor the fixed-point one decided */
     int64_t near_ties;           /* FP64 |p - alpha| < 1e-12 (decision could differ from any other FP64 order) */
     int64_t large_tests;         /* tests counted in global memory */
     double max_abs_dp;           /* max |p32 - p64| over rechecked tests */
     double count_ms;             /* device time of the shared-memory counting+scoring kernel (CUDA events) */
-    double count_bytes;          /* algorithmic bytes its tests read: sum (2+d) * n_samples */
+    double count_bytes;          /* algorithmic bytes its tests read: sum (2+d) * n_samples over the
+                                    tests not decided without a count */
     double large_ms;             /* device time of the global-memory (large table) kernel */
     int64_t count_launches;      /* launches of the counting+scoring kernels */
     int64_t kernel_launches;     /* launches of this library's own kernels (library scans excluded) */
