@@ -78,6 +78,7 @@ int dev_alloc(void **p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) {
         *p = nullptr;
+        cudaGetLastError();  // reported here: a caller that does without must not meet it at its next launch
         return set_error(FPGM_ERR_OOM, "cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
     }
     std::lock_guard<std::mutex> lk(g_alloc_mu);
