@@ -220,6 +220,7 @@ struct fpgm_engine {
     // wave log keep them on the per-test kernels)
     bool strata_on = true, strata_ready = false;
     bool strata_level = false;          // this level's waves use them
+    bool strata_short = false;          // no room for them in this skeleton
     DevBuf strata_tab, strata_lists, strata_pool, strata_refs, strata_used;
     // fixed-point statistic (fixed.cuh) and tables per variable set (sets.cuh; FPGM_SETS=0: none)
     DevBuf fixed_f, tight;
@@ -1399,7 +1400,7 @@ void strata_args(fpgm_engine *e, StrataArgs &s) {
 int strata_setup(fpgm_engine *e, int d, bool first, const unsigned long long *last_used) {
     e->strata_level = false;
     if (first) e->strata_ready = false;
-    if (!e->strata_on || !e->wide_on || e->wave_log || e->phase_timers.p || e->fixed_n < e->S || d < 1 ||
+    if (!e->strata_on || e->strata_short || !e->wide_on || e->wave_log || e->phase_timers.p || e->fixed_n < e->S || d < 1 ||
         d + 1 > kStrataMaxSets || max_table_ints(e->h_card, d) <= kCtaInts - 64)
         return FPGM_OK;
     const size_t tab = kStrataKeyBytes + (size_t)kStrataNodes * 24 + (size_t)kStrataPairs * 16;
@@ -1420,7 +1421,7 @@ int strata_setup(fpgm_engine *e, int d, bool first, const unsigned long long *la
             e->strata_pool.release();
             empty = true;
             if (e->strata_pool.ensure(want) != FPGM_OK && e->strata_pool.ensure(least) != FPGM_OK) {
-                e->strata_on = false;  // no room: the per-test kernels
+                e->strata_short = true;  // no room: the per-test kernels
                 return FPGM_OK;
             }
         }
@@ -1429,7 +1430,9 @@ int strata_setup(fpgm_engine *e, int d, bool first, const unsigned long long *la
     if (e->strata_tab.ensure(tab) != FPGM_OK ||
         e->strata_lists.ensure(((size_t)(kStrataMaxSets + 1) * kStrataBuild + kStrataPairs) * 4) != FPGM_OK ||
         e->strata_used.ensure(64 + sizeof(StrataCounters)) != FPGM_OK) {
-        e->strata_on = false;
+        e->strata_short = true;
+        e->strata_ready = false;
+        e->strata_pool.release();
         return FPGM_OK;
     }
     if (empty) {
@@ -1967,6 +1970,7 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
         }
     } live_scope(e);
     e->in_skeleton = true;
+    e->strata_short = false;
     RET(fixed_setup(e));
     if (e->live_on) {  // contributing-sample counts, measured level by level
         RET(e->live_stat.ensure(16));
