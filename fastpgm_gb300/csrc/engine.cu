@@ -63,12 +63,17 @@ size_t g_alloc_bytes = 0;
 }  // namespace
 
 namespace fpgm {
-int dev_alloc(void **p, size_t bytes) {
-    *p = nullptr;
+static size_t alloc_cap() {
     static const size_t cap = [] {
         const char *c = getenv("FPGM_DEVICE_MEM_CAP");
         return c ? (size_t)strtoull(c, nullptr, 10) : (size_t)0;
     }();
+    return cap;
+}
+
+int dev_alloc(void **p, size_t bytes) {
+    *p = nullptr;
+    const size_t cap = alloc_cap();
     {
         std::lock_guard<std::mutex> lk(g_alloc_mu);
         if (cap && g_alloc_bytes + bytes > cap)
@@ -91,6 +96,18 @@ void dev_free(void *p, size_t bytes) {
     cudaFree(p);
     std::lock_guard<std::mutex> lk(g_alloc_mu);
     g_alloc_bytes -= std::min(bytes, g_alloc_bytes);
+}
+
+// Bytes that dev_alloc can still hand out on the current device.
+static size_t dev_room() {
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    const size_t cap = alloc_cap();
+    std::lock_guard<std::mutex> lk(g_alloc_mu);
+    return cap ? std::min(free_b, cap > g_alloc_bytes ? cap - g_alloc_bytes : 0) : free_b;
 }
 }  // namespace fpgm
 
@@ -221,6 +238,8 @@ struct fpgm_engine {
     bool strata_on = true, strata_ready = false;
     bool strata_level = false;          // this level's waves use them
     bool strata_short = false;          // no room for them in this skeleton
+    int given_back = 0;                 // times that give_back released the optional memory
+    bool spare = true;                  // ... not yet in this skeleton
     DevBuf strata_tab, strata_lists, strata_pool, strata_refs, strata_used;
     // fixed-point statistic (fixed.cuh) and tables per variable set (sets.cuh; FPGM_SETS=0: none)
     DevBuf fixed_f, tight;
@@ -251,6 +270,30 @@ struct fpgm_engine {
 
 // ------------------------------------------------------------------ kernels
 namespace {
+
+// ---- memory
+// What a skeleton can do without (set tables, shared strata, the bounds' statistics) stays with the engine
+// from one call to the next.  It is given back when something that a call cannot do without finds
+// no room; the rest of the skeleton counts test by test.
+bool give_back(fpgm_engine *e) {
+    DevBuf *bufs[] = {&e->strata_pool, &e->strata_tab, &e->strata_lists, &e->strata_refs, &e->set_pool, &e->set_tab,
+                      &e->set_items,   &e->tri_tab,    &e->tri_g,        &e->pair_g2};
+    size_t held = 0;
+    for (DevBuf *b : bufs) held += b->bytes;
+    if (held == 0) return false;
+    cudaStreamSynchronize(e->stream);  // the launches that use it are done
+    for (DevBuf *b : bufs) b->release();
+    e->strata_level = e->strata_ready = e->sets_level = e->tri_ready = e->pairs_kept = false;
+    e->spare = false;
+    ++e->given_back;
+    return true;
+}
+// A buffer that the call cannot do without.
+int need(fpgm_engine *e, DevBuf &b, size_t bytes, bool keep = false) {
+    int rc = b.ensure(bytes, keep, e->stream);
+    if (rc == FPGM_ERR_OOM && give_back(e)) rc = b.ensure(bytes, keep, e->stream);
+    return rc;
+}
 
 // ---- data preparation
 // First-appearance ids per column (Dataset.cpp:459-467) and observed cardinality: a cluster of
@@ -929,7 +972,7 @@ int load_tune_table(fpgm_engine *e) {
     }
     fclose(f);
     if (!entries) return FPGM_OK;
-    RET(e->tune.ensure(t.size()));
+    RET(need(e, e->tune, t.size()));
     CK(cudaMemcpy(e->tune.p, t.data(), t.size(), cudaMemcpyHostToDevice));
     e->tune_loaded = true;
     e->tune_source = path;
@@ -994,11 +1037,11 @@ extern "C" int fpgm_engine_create(int32_t device, fpgm_engine **out) {
             bt[(size_t)n * kBinomK + k] = (s < a || a == ~0ull || b == ~0ull) ? ~0ull : s;
         }
     }
-    RET(e->btab.ensure(bt.size() * 8));
+    RET(need(e, e->btab, bt.size() * 8));
     CK(cudaMemcpy(e->btab.p, bt.data(), bt.size() * 8, cudaMemcpyHostToDevice));
-    RET(e->counters.ensure(kCounterBytes));
+    RET(need(e, e->counters, kCounterBytes));
     CK(cudaHostAlloc(reinterpret_cast<void **>(&e->level_host), 1024, cudaHostAllocDefault));
-    RET(e->stats.ensure(ST_COUNT * 8));
+    RET(need(e, e->stats, ST_COUNT * 8));
     e->wave_log = getenv("FPGM_WAVE_LOG") != nullptr;
     if (const char *pm = getenv("FPGM_PART_MAX_LOG")) e->part_max_log = std::min(kPartMaxLog, std::max(1, atoi(pm)));
     if (const char *w = getenv("FPGM_WIDE")) e->wide_on = atoi(w) != 0;
@@ -1021,7 +1064,7 @@ extern "C" int fpgm_engine_create(int32_t device, fpgm_engine **out) {
     if (const char *w = getenv("FPGM_TUNE")) e->tune_online = e->tune_online && atoi(w) != 0;
     RET(load_tune_table(e));
     if (e->tune_online && !e->tune_loaded) {
-        RET(e->tune_obs.ensure((size_t)kTuneBuckets * 8 * 8));
+        RET(need(e, e->tune_obs, (size_t)kTuneBuckets * 8 * 8));
         CK(cudaMemset(e->tune_obs.p, 0, (size_t)kTuneBuckets * 8 * 8));
     }
     if (const char *w = getenv("FPGM_OVF_SKIP")) e->ovf_on = atoi(w) != 0;
@@ -1030,11 +1073,11 @@ extern "C" int fpgm_engine_create(int32_t device, fpgm_engine **out) {
     if (const char *w = getenv("FPGM_LIVE_MIN_LEVEL")) e->live_min_level = std::max(1, atoi(w));
     if (const char *w = getenv("FPGM_LIVE_FRAC")) e->live_frac = atof(w);
     if (e->ovf_on) {
-        RET(e->ovf.ensure((size_t)kTuneBuckets * 8 * 8));
+        RET(need(e, e->ovf, (size_t)kTuneBuckets * 8 * 8));
         CK(cudaMemset(e->ovf.p, 0, (size_t)kTuneBuckets * 8 * 8));
     }
     if (getenv("FPGM_PHASE_TIMERS")) {
-        RET(e->phase_timers.ensure(32 * 8));
+        RET(need(e, e->phase_timers, 32 * 8));
         CK(cudaMemset(e->phase_timers.p, 0, 32 * 8));
     }
     *out = e;
@@ -1097,8 +1140,8 @@ int load_datasets(fpgm_engine *e, int32_t n_jobs, const int32_t *job_vars, const
     e->h_var_S.resize(n);
     e->h_var_lo.resize(n);
     e->h_var_hi.resize(n);
-    RET(e->cols.ensure((size_t)bytes + 64));
-    RET(e->card.ensure(std::max<size_t>(256, (size_t)n)));
+    RET(need(e, e->cols, (size_t)bytes + 64));
+    RET(need(e, e->card, std::max<size_t>(256, (size_t)n)));
     CK(cudaMemsetAsync(e->cols.p, 0, (size_t)bytes, e->stream));
     int64_t off = 0;
     int32_t v0 = 0;
@@ -1115,10 +1158,10 @@ int load_datasets(fpgm_engine *e, int32_t n_jobs, const int32_t *job_vars, const
         off += job_vars[j] * pitch;
         v0 += job_vars[j];
     }
-    RET(e->var_off.ensure((size_t)n * 8));
-    RET(e->var_S.ensure((size_t)n * 4));
-    RET(e->var_lo.ensure((size_t)n * 4));
-    RET(e->var_hi.ensure((size_t)n * 4));
+    RET(need(e, e->var_off, (size_t)n * 8));
+    RET(need(e, e->var_S, (size_t)n * 4));
+    RET(need(e, e->var_lo, (size_t)n * 4));
+    RET(need(e, e->var_hi, (size_t)n * 4));
     CK(cudaMemcpyAsync(e->var_off.p, e->h_var_off.data(), (size_t)n * 8, cudaMemcpyHostToDevice, e->stream));
     CK(cudaMemcpyAsync(e->var_S.p, e->h_var_S.data(), (size_t)n * 4, cudaMemcpyHostToDevice, e->stream));
     CK(cudaMemcpyAsync(e->var_lo.p, e->h_var_lo.data(), (size_t)n * 4, cudaMemcpyHostToDevice, e->stream));
@@ -1186,7 +1229,7 @@ int ensure_quantiles(fpgm_engine *e, DevBuf &buf, double &have_alpha, int &have_
     while (n < df && n < kBandDfMax) n <<= 1;
     if (have_alpha == alpha && buf.p && n <= have_df) return FPGM_OK;
     have_alpha = -1.0;
-    RET(buf.ensure((size_t)2 * (n + 1) * sizeof(double)));
+    RET(need(e, buf, (size_t)2 * (n + 1) * sizeof(double)));
     double *lo = buf.as<double>(), *hi = lo + n + 1;
     band_table_kernel<<<blocks_for(2 * (n + 1), 64), 64, 0, e->stream>>>(alpha, band, lo, hi, n);
     CK(cudaGetLastError());
@@ -1226,10 +1269,10 @@ int ensure_slots(fpgm_engine *e) {
     e->hash_cap_global = (int)cap;
     e->n_slots = 2 * e->num_sms;
     e->slot_bytes = slot_layout(e->slot_S, cap).total;
-    RET(e->slots.ensure((size_t)e->slot_bytes * e->n_slots));
+    RET(need(e, e->wide, (size_t)e->n_slots * sizeof(WideTest)));  // before the slots, whose presence stands for all
+    RET(need(e, e->wide_items, (size_t)e->n_slots * kPartMax * 4));
+    RET(need(e, e->slots, (size_t)e->slot_bytes * e->n_slots));
     CK(cudaMemsetAsync(e->slots.p, 0, (size_t)e->slot_bytes * e->n_slots, e->stream));  // zeroed tables
-    RET(e->wide.ensure((size_t)e->n_slots * sizeof(WideTest)));
-    RET(e->wide_items.ensure((size_t)e->n_slots * kPartMax * 4));
     return FPGM_OK;
 }
 
@@ -1271,7 +1314,7 @@ int live_setup(fpgm_engine *e, int d) {
                 return FPGM_OK;
             }
         }
-        RET(e->live_cnt.ensure(16));
+        RET(need(e, e->live_cnt, 16));
         e->live_cap = cap;
         e->live_tab_cap = tcap;
         e->live_words = (int32_t)words;
@@ -1290,7 +1333,7 @@ void launch_warp_tier(fpgm_engine *e, const WaveArgs &a);
 int fixed_setup(fpgm_engine *e) {
     if (e->S > kFixedMaxSamples || e->fixed_n >= e->S) return FPGM_OK;
     e->fixed_n = 0;
-    RET(e->fixed_f.ensure((size_t)(e->S + 1) * 8));
+    RET(need(e, e->fixed_f, (size_t)(e->S + 1) * 8));
     const double top = (double)e->S * log((double)std::max<int64_t>(e->S, 3));
     const int k = 59 - (int)ceil(log2(top));  // four sums of at most `top` stay below 2^61
     fixed_table_kernel<<<blocks_for(e->S + 1, 256), 256, 0, e->stream>>>(e->fixed_f.as<long long>(), e->S, ldexp(1.0, k));
@@ -1307,7 +1350,7 @@ int fixed_setup(fpgm_engine *e) {
 constexpr size_t kSetPoolMax = (size_t)4 << 30;
 int sets_setup(fpgm_engine *e, int d, int64_t n_active) {
     e->sets_level = false;
-    if (!e->sets_on || e->fixed_n < e->S || e->wave_log || e->phase_timers.p) return FPGM_OK;
+    if (!e->sets_on || !e->spare || e->fixed_n < e->S || e->wave_log || e->phase_timers.p) return FPGM_OK;
     const int64_t tests = std::min<int64_t>(e->level_tests, 64 * n_active);
     int32_t cap = 1 << 12;
     while (cap < 4 * tests && cap < (1 << 22)) cap <<= 1;
@@ -1396,38 +1439,39 @@ void strata_args(fpgm_engine *e, StrataArgs &s) {
 }
 
 // Level d's waves count through shared strata when a test can go past shared memory: buffers
-// made (or, when the last level came near their end, grown and emptied).  No room: not used.
+// made (or, when the last level came near their end, grown and emptied).  The pool takes room for
+// 8,192 sets and 256 MB at least, more when a level used half of it, but not more than a quarter of
+// the memory that is left (the per-test kernels' slots have theirs by now) nor, past the 256 MB,
+// than the level's tests can fill.  No room: not used in this skeleton.
 int strata_setup(fpgm_engine *e, int d, bool first, const unsigned long long *last_used) {
     e->strata_level = false;
     if (first) e->strata_ready = false;
-    if (!e->strata_on || e->strata_short || !e->wide_on || e->wave_log || e->phase_timers.p || e->fixed_n < e->S || d < 1 ||
-        d + 1 > kStrataMaxSets || max_table_ints(e->h_card, d) <= kCtaInts - 64)
+    if (!e->strata_on || !e->spare || e->strata_short || !e->wide_on || e->wave_log || e->phase_timers.p || e->fixed_n < e->S ||
+        d < 1 || d + 1 > kStrataMaxSets || max_table_ints(e->h_card, d) <= kCtaInts - 64)
         return FPGM_OK;
     const size_t tab = kStrataKeyBytes + (size_t)kStrataNodes * 24 + (size_t)kStrataPairs * 16;
-    const size_t slot = (size_t)((e->S + 15) & ~(int64_t)15) * 2;
+    const size_t slot = (size_t)((e->S + 15) & ~(int64_t)15) * 2, floor = (size_t)256 << 20;
     unsigned long long used[3] = {0, 0, 0};  // at the end of the last level
     if (e->strata_ready) memcpy(used, last_used, sizeof used);
     bool empty = !e->strata_ready;
-    const size_t least = std::max<size_t>((size_t)256 << 20, slot * 8192);
-    size_t want = std::max(least, e->strata_pool.bytes);
+    size_t want = std::max(std::max(floor, slot * 8192), e->strata_pool.bytes);
     if (e->strata_ready && used[0] > e->strata_pool.bytes / 2) want = std::max(want, 4 * e->strata_pool.bytes);
-    if (e->strata_pool_fixed) {
-        if (!e->strata_pool.p) RET(e->strata_pool.ensure(e->strata_pool_fixed));
-    } else if (want > e->strata_pool.bytes) {
-        size_t free_b = 0, total_b = 0;
-        CK(cudaMemGetInfo(&free_b, &total_b));
-        want = std::min(want, std::max(least, (size_t)std::min(32.0e9, 0.25 * (double)(free_b + e->strata_pool.bytes))));
+    // a test enters at most d + d + 1 sets, and two pairs of a byte per stratum
+    const double most = (double)e->level_tests * ((2.0 * d + 1.0) * (double)slot + 131072.0);
+    want = std::max(floor, (size_t)std::min((double)want, most));
+    if (e->strata_pool_fixed) want = e->strata_pool_fixed;
+    bool ok = true;
+    if (want > e->strata_pool.bytes) {
+        if (!e->strata_pool_fixed)
+            want = std::min(want, (size_t)std::min(32.0e9, 0.25 * (double)(dev_room() + e->strata_pool.bytes)));
         if (want > e->strata_pool.bytes + e->strata_pool.bytes / 4) {
             e->strata_pool.release();
             empty = true;
-            if (e->strata_pool.ensure(want) != FPGM_OK && e->strata_pool.ensure(least) != FPGM_OK) {
-                e->strata_short = true;  // no room: the per-test kernels
-                return FPGM_OK;
-            }
+            ok = (e->strata_pool_fixed || want >= slot * 64) && e->strata_pool.ensure(want) == FPGM_OK;
         }
     }
     if (used[0] > e->strata_pool.bytes / 2 || used[1] > kStrataNodes / 3 || used[2] > kStrataPairs / 3) empty = true;
-    if (e->strata_tab.ensure(tab) != FPGM_OK ||
+    if (!ok || e->strata_tab.ensure(tab) != FPGM_OK ||
         e->strata_lists.ensure(((size_t)(kStrataMaxSets + 1) * kStrataBuild + kStrataPairs) * 4) != FPGM_OK ||
         e->strata_used.ensure(64 + sizeof(StrataCounters)) != FPGM_OK) {
         e->strata_short = true;
@@ -1458,7 +1502,7 @@ int launch_strata(fpgm_engine *e, const WaveArgs &a) {
     return a.d + 5;
 }
 
-int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t items) {
+int wave_args_fill(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t items) {
     memset(&a, 0, sizeof a);
     a.cols = e->cols.as<uint8_t>();
     a.var_off = e->var_off.as<int64_t>();
@@ -1486,9 +1530,9 @@ int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t ite
         a.fx.hi = a.fx.lo + e->tight_df + 1;
         a.fx.dfmax = e->tight_df;
     }
-    RET(e->item_vars.ensure((size_t)std::max<int64_t>(items, 1) * (2 + d) * 2 + 16));
-    RET(e->lists.ensure((size_t)7 * std::max<int64_t>(items, 1) * 4 + 16));
-    RET(e->flag.ensure((size_t)std::max<int64_t>(items, 1) + 16));
+    RET(need(e, e->item_vars, (size_t)std::max<int64_t>(items, 1) * (2 + d) * 2 + 16));
+    RET(need(e, e->lists, (size_t)7 * std::max<int64_t>(items, 1) * 4 + 16));
+    RET(need(e, e->flag, (size_t)std::max<int64_t>(items, 1) + 16));
     a.item_vars = e->item_vars.as<uint16_t>();
     a.lists = e->lists.as<int32_t>();
     a.list_cap = std::max<int64_t>(items, 1);
@@ -1543,7 +1587,6 @@ int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t ite
     }
     if (e->sets_level) {
         const size_t ni = (size_t)std::max<int64_t>(items, 1);
-        RET(e->set_items.ensure(ni * 6 * sizeof(int2)));
         a.sets.used = e->set_tab.as<unsigned long long>();
         a.sets.key = reinterpret_cast<uint64_t *>(e->set_tab.as<char>() + 16);
         a.sets.cap = e->sets_cap;
@@ -1556,15 +1599,23 @@ int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t ite
         a.sets.fresh = a.sets.items + ni;
         a.sets.few = 6 * e->num_sms;
     }
-    if (e->strata_level && d >= 1) {
-        RET(e->strata_refs.ensure((size_t)std::max<int64_t>(items, 1) * (2 * sizeof(int4) + 8)));
-        a.strata_card = kStrataMaxCard;
-    }
+    if (e->strata_level && d >= 1) a.strata_card = kStrataMaxCard;
     a.part_max_log = e->part_max_log;
     a.warp_ints = e->warp_small ? kWarpIntsSmall : kWarpInts;
     a.dense_rows = e->dense_rows;
     a.stage_rec = e->stage_rec;
     return FPGM_OK;
+}
+
+int wave_args_base(fpgm_engine *e, WaveArgs &a, double alpha, int d, int64_t items) {
+    const size_t ni = (size_t)std::max<int64_t>(items, 1);
+    if (e->sets_level && e->set_items.ensure(ni * 6 * sizeof(int2)) != FPGM_OK) e->sets_level = false;
+    if (e->strata_level && d >= 1 && e->strata_refs.ensure(ni * (2 * sizeof(int4) + 8)) != FPGM_OK) e->strata_level = false;
+    for (;;) {  // again when a buffer's room came from memory that the arguments point into
+        const int before = e->given_back;
+        RET(wave_args_fill(e, a, alpha, d, items));
+        if (e->given_back == before) return FPGM_OK;
+    }
 }
 
 // Level 2's bounds (triple_enter_kernel), before its waves and before its own set table takes
@@ -1584,6 +1635,7 @@ int triples_setup(fpgm_engine *e, double alpha, const WaveArgs &proto, int64_t n
     if (e->tri_g.ensure(g_bytes + (size_t)e->sets_cap * 4) != FPGM_OK) return FPGM_OK;
     WaveArgs a;
     RET(wave_args_base(e, a, alpha, 1, items));
+    if (!e->sets_level) return FPGM_OK;  // no room for its lists, or level 1's sets were given back
     a.adjl = proto.adjl;
     a.adj_stride = proto.adj_stride;
     a.deg = proto.deg;
@@ -1711,6 +1763,12 @@ int run_waves_graph(fpgm_engine *e, double alpha, int d, int64_t n_active, int64
                     const WaveArgs &proto, PendingLevel &pend) {
     // items of one wave at most
     const int64_t cap = std::max<int64_t>(n_active, std::min<int64_t>(kMaxItems, std::max<int64_t>(e->level_tests, 1 << 16)));
+    if (n_active > kBeginEdges) {
+        size_t sb = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, sb, e->g.as<int32_t>(), e->off.as<int32_t>(), (int)(n_active + 1),
+                                      e->stream);
+        RET(need(e, e->scan_tmp, sb + 16));
+    }
     WaveArgs a = proto;
     RET(wave_args_base(e, a, alpha, d, cap));
     a.adjl = proto.adjl;
@@ -1725,12 +1783,6 @@ int run_waves_graph(fpgm_engine *e, double alpha, int d, int64_t n_active, int64
     a.off = e->off.as<int32_t>();
     a.n_edges = (int32_t)n_active;
     a.dbg = nullptr;
-    if (n_active > kBeginEdges) {
-        size_t sb = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, sb, e->g.as<int32_t>(), e->off.as<int32_t>(), (int)(n_active + 1),
-                                      e->stream);
-        RET(e->scan_tmp.ensure(sb + 16));
-    }
     pend.device = true;
     // the first wave's share of every edge (wave_begin's rule; edges without ranks only raise it)
     const int64_t q0 = std::min<int64_t>(std::min<int64_t>(4096, (e->ci_blocks * 64ll + n_active - 1) / n_active),
@@ -1837,7 +1889,7 @@ int run_waves_and_count(fpgm_engine *e, double alpha, int d, int64_t n_active, f
     size_t scan_bytes = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, e->g.as<int32_t>(), e->off.as<int32_t>(),
                                   (int)(n_active + 1), e->stream);
-    RET(e->scan_tmp.ensure(scan_bytes + 16));
+    RET(need(e, e->scan_tmp, scan_bytes + 16));
     while (unresolved > 0) {
         int64_t q = (int64_t)1 << std::min(wave, 12);
         const int64_t target = (int64_t)e->ci_blocks * 64;
@@ -1970,25 +2022,26 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
         }
     } live_scope(e);
     e->in_skeleton = true;
+    e->spare = true;
     e->strata_short = false;
     RET(fixed_setup(e));
     if (e->live_on) {  // contributing-sample counts, measured level by level
-        RET(e->live_stat.ensure(16));
+        RET(need(e, e->live_stat, 16));
         CK(cudaMemsetAsync(e->live_stat.p, 0, 16, e->stream));
         e->live_prev[0] = e->live_prev[1] = 0ull;
         e->live_next = false;
     }
-    RET(e->bits.ensure((size_t)n * W * 4));
+    RET(need(e, e->bits, (size_t)n * W * 4));
     init_bits_kernel<<<blocks_for((int64_t)n * W, 256), 256, 0, e->stream>>>(
         e->bits.as<uint32_t>(), n, W, e->var_lo.as<int32_t>(), e->var_hi.as<int32_t>());
     CK(cudaGetLastError());
     st->kernel_launches += 1;
-    RET(e->log_pair.ensure((size_t)E * 8 + 16));
-    RET(e->log_meta.ensure((size_t)E * 8 + 16));
-    RET(e->log_vars.ensure((size_t)1 << 20));
-    RET(e->deg.ensure((size_t)n * 4 + 16));
-    RET(e->node_cnt.ensure((size_t)(n + 1) * 4));
-    RET(e->node_off.ensure((size_t)(n + 1) * 4));
+    RET(need(e, e->log_pair, (size_t)E * 8 + 16));
+    RET(need(e, e->log_meta, (size_t)E * 8 + 16));
+    RET(need(e, e->log_vars, (size_t)1 << 20));
+    RET(need(e, e->deg, (size_t)n * 4 + 16));
+    RET(need(e, e->node_cnt, (size_t)(n + 1) * 4));
+    RET(need(e, e->node_off, (size_t)(n + 1) * 4));
     int64_t log_count = 0, var_count = 0;
     int max_deg = 0;  // largest dataset - 1
     for (int v = 0; v < n; ++v) max_deg = std::max(max_deg, e->h_var_hi[v] - e->h_var_lo[v] - 1);
@@ -2005,21 +2058,21 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
         const bool snap = !complete && d >= 1 && n <= kSnapNodes;  // the level's start in one launch
         int stride = 1;
         const size_t ne = (size_t)std::max<int64_t>(n_active, 1) + 1;
-        RET(e->edges_x.ensure(ne * 4));
-        RET(e->edges_y.ensure(ne * 4));
-        RET(e->pxy.ensure(ne * 4));
-        RET(e->pyx.ensure(ne * 4));
-        RET(e->cntx.ensure(ne * 8));
-        RET(e->total.ensure(ne * 8));
-        RET(e->next.ensure(ne * 8));
-        RET(e->seprank.ensure(ne * 8));
-        RET(e->status.ensure(ne));
-        RET(e->g.ensure(ne * 4));
-        RET(e->off.ensure(ne * 4));
-        RET(e->wave_ctl.ensure(sizeof(WaveCtl)));
+        RET(need(e, e->edges_x, ne * 4));
+        RET(need(e, e->edges_y, ne * 4));
+        RET(need(e, e->pxy, ne * 4));
+        RET(need(e, e->pyx, ne * 4));
+        RET(need(e, e->cntx, ne * 8));
+        RET(need(e, e->total, ne * 8));
+        RET(need(e, e->next, ne * 8));
+        RET(need(e, e->seprank, ne * 8));
+        RET(need(e, e->status, ne));
+        RET(need(e, e->g, ne * 4));
+        RET(need(e, e->off, ne * 4));
+        RET(need(e, e->wave_ctl, sizeof(WaveCtl)));
         if (!complete) {  // the level's snapshot (several datasets: also at level 0)
             stride = std::max(1, max_deg);
-            RET(e->adjl.ensure((size_t)n * stride * 4));
+            RET(need(e, e->adjl, (size_t)n * stride * 4));
         }
         if (!complete && !snap) {
             csr_kernel<<<blocks_for(n, 128), 128, 0, e->stream>>>(e->bits.as<uint32_t>(), n, W, e->adjl.as<int32_t>(),
@@ -2031,7 +2084,7 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
             size_t sb = 0;
             cub::DeviceScan::ExclusiveSum(nullptr, sb, e->node_cnt.as<int32_t>(), e->node_off.as<int32_t>(), n + 1,
                                           e->stream);
-            RET(e->scan_tmp.ensure(sb + 16));
+            RET(need(e, e->scan_tmp, sb + 16));
             sb = e->scan_tmp.bytes;
             CK(cub::DeviceScan::ExclusiveSum(e->scan_tmp.p, sb, e->node_cnt.as<int32_t>(), e->node_off.as<int32_t>(),
                                              n + 1, e->stream));
@@ -2085,8 +2138,14 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
             bool gram = false;
             if (d == 0 && e->n_jobs == 1 && e->gram_on) {
                 if (!e->gram_planned) {
-                    RET(gram_plan(e->gram, n, e->h_card.data(), e->S, e->cols.as<uint8_t>(), e->var_off.as<int64_t>(),
-                                  e->card.as<uint8_t>(), e->num_sms, e->stream, &e->gram_ok));
+                    auto plan = [&] {
+                        return gram_plan(e->gram, n, e->h_card.data(), e->S, e->cols.as<uint8_t>(),
+                                         e->var_off.as<int64_t>(), e->card.as<uint8_t>(), e->num_sms, e->stream,
+                                         &e->gram_ok);
+                    };
+                    int rc = plan();
+                    if (rc == FPGM_ERR_OOM && give_back(e)) rc = plan();
+                    RET(rc);
                     e->gram_planned = true;
                     if (e->gram_ok) {
                         int occ = 0;
@@ -2097,8 +2156,10 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
                 }
                 gram = e->gram_ok;
             }
+            // what the level cannot do without comes before the pools that take their share of the rest
+            if (max_table_ints(e->h_card, d) > kCtaInts - 64) RET(ensure_slots(e));
             if (d == 0) {  // every pair's statistic is kept when level 0 computes it in fixed point
-                e->pairs_kept = e->bound_on && e->fixed_n >= e->S && n <= kPairVars && !e->wave_log &&
+                e->pairs_kept = e->bound_on && e->spare && e->fixed_n >= e->S && n <= kPairVars && !e->wave_log &&
                                 !e->phase_timers.p && (gram || (e->sets_on && e->n_jobs > 1)) &&
                                 max_table_ints(e->h_card, 0) * 2 <= kCtaInts &&
                                 e->pair_g2.ensure((size_t)n * n * sizeof(float)) == FPGM_OK;
@@ -2120,8 +2181,7 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
                 RET(run_waves_and_count(e, alpha, d, n_active, st, st->n_levels, a));
         }
         // finalize: removals into the bitset and the removal log
-        RET(e->log_vars.ensure((size_t)(var_count + std::max<int64_t>(n_active, 1) * std::max(d, 1)) * 4 + 16, true,
-                               e->stream));
+        RET(need(e, e->log_vars, (size_t)(var_count + std::max<int64_t>(n_active, 1) * std::max(d, 1)) * 4 + 16, true));
         if (var_count + n_active * (int64_t)d > INT32_MAX)
             return set_error(FPGM_ERR_UNSUPPORTED, "separating-set storage beyond 2^31 entries");
         const bool one = n_active <= 16384 && (int64_t)n * W <= 32768;  // removals and degrees in one CTA
@@ -2205,18 +2265,18 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
     // result, assembled on the device: the 0/1 adjacency expanded from the bitset, and the
     // removal log sorted by pair (a < b, ascending) with each separating set gathered in that
     // order; the host only copies it back
-    RET(e->res_adj_d.ensure((size_t)n * n + 16));
+    RET(need(e, e->res_adj_d, (size_t)n * n + 16));
     expand_adj_kernel<<<blocks_for((int64_t)n * n, 256), 256, 0, e->stream>>>(e->bits.as<uint32_t>(), n, W,
                                                                              e->res_adj_d.as<uint8_t>());
     CK(cudaGetLastError());
     st->kernel_launches += 1;
     const int R = (int)log_count;
     if (R > 0) {
-        RET(e->res_key.ensure((size_t)R * 4 * 2 + 16));
-        RET(e->res_idx.ensure((size_t)R * 4 * 2 + 16));
-        RET(e->res_removed_d.ensure((size_t)R * 8 + 16));
-        RET(e->res_cnt.ensure((size_t)(R + 1) * 4 * 2 + 16));
-        RET(e->res_vars_d.ensure((size_t)var_count * 4 + 16));
+        RET(need(e, e->res_key, (size_t)R * 4 * 2 + 16));
+        RET(need(e, e->res_idx, (size_t)R * 4 * 2 + 16));
+        RET(need(e, e->res_removed_d, (size_t)R * 8 + 16));
+        RET(need(e, e->res_cnt, (size_t)(R + 1) * 4 * 2 + 16));
+        RET(need(e, e->res_vars_d, (size_t)var_count * 4 + 16));
         uint32_t *k0 = e->res_key.as<uint32_t>(), *k1 = k0 + R;
         int32_t *i0 = e->res_idx.as<int32_t>(), *i1 = i0 + R;
         int32_t *cnt = e->res_cnt.as<int32_t>(), *off = cnt + R + 1;
@@ -2228,7 +2288,7 @@ int run_batched(fpgm_engine *e, double alpha, int depth, fpgm_pc_stats *st) {
         CK(cub::DeviceRadixSort::SortPairs(nullptr, sb, k0, k1, i0, i1, R, 0, bits, e->stream));
         size_t sb2 = 0;
         CK(cub::DeviceScan::ExclusiveSum(nullptr, sb2, cnt, off, R + 1, e->stream));
-        RET(e->scan_tmp.ensure(std::max(sb, sb2) + 16));
+        RET(need(e, e->scan_tmp, std::max(sb, sb2) + 16));
         sb = e->scan_tmp.bytes;
         CK(cub::DeviceRadixSort::SortPairs(e->scan_tmp.p, sb, k0, k1, i0, i1, R, 0, bits, e->stream));
         log_gather_kernel<<<blocks_for(R + 1, 256), 256, 0, e->stream>>>(R, i1, e->log_pair.as<int32_t>(),
@@ -2273,10 +2333,10 @@ int plain_grid(const fpgm_engine *e, int64_t S) {
 int plain_test(fpgm_engine *e, int x, int y, const int *z, int d, double alpha, int want_hash,
                fpgm_ci_result *out, fpgm_pc_stats *st = nullptr) {
     if (!e->plain_ws.p) {
-        RET(e->plain_ws.ensure((size_t)kPlainInts * 4 + 64));
+        RET(need(e, e->plain_ws, (size_t)kPlainInts * 4 + 64));
         CK(cudaMemsetAsync(e->plain_ws.p, 0, e->plain_ws.bytes, e->stream));
     }
-    RET(e->detail_buf.ensure(sizeof(fpgm_ci_result) * 64));
+    RET(need(e, e->detail_buf, sizeof(fpgm_ci_result) * 64));
     // table size decides: dense grid-wide kernel, or the compact-strata kernel on one CTA
     double cells = (double)e->h_card[x] * e->h_card[y], dz = 1.0;
     for (int k = 0; k < d; ++k) dz *= e->h_card[z[k]];
@@ -2650,9 +2710,9 @@ extern "C" int fpgm_mle_cpts(fpgm_engine *e, const int32_t *parent_off, const in
     memcpy(meta.data(), nodes.data(), sizeof(MleNode) * n);
     if (parent_off[n] > 0) memcpy(meta.data() + par_at, parents, (size_t)parent_off[n] * 4);
     if (!large.empty()) memcpy(meta.data() + large_at, large.data(), large.size() * 4);
-    RET(e->mle_meta.ensure(meta.size()));
-    RET(e->mle_counts.ensure((size_t)(total + n) * 4));
-    RET(e->mle_pot.ensure((size_t)total * 8 + 16));
+    RET(need(e, e->mle_meta, meta.size()));
+    RET(need(e, e->mle_counts, (size_t)(total + n) * 4));
+    RET(need(e, e->mle_pot, (size_t)total * 8 + 16));
     CK(cudaMemcpyAsync(e->mle_meta.p, meta.data(), meta.size(), cudaMemcpyHostToDevice, e->stream));
     CK(cudaMemsetAsync(e->mle_counts.p, 0, (size_t)(total + n) * 4, e->stream));
     // slices per node: enough CTAs to fill the GPU, at least 64 vectors each
@@ -2716,8 +2776,8 @@ extern "C" int fpgm_ci_test_batch(fpgm_engine *e, const int32_t *tests, int32_t 
             if (e->h_var_lo[tests[t * (2 + d) + k]] != e->h_var_lo[tests[t * (2 + d)]])
                 return set_error(FPGM_ERR_INVALID, "fpgm_ci_test_batch: test %lld mixes datasets", (long long)t);
     CK(cudaSetDevice(e->device));
-    RET(e->tests_buf.ensure((size_t)n_tests * (2 + d) * 4));
-    RET(e->detail_buf.ensure((size_t)n_tests * sizeof(fpgm_ci_result)));
+    RET(need(e, e->tests_buf, (size_t)n_tests * (2 + d) * 4));
+    RET(need(e, e->detail_buf, (size_t)n_tests * sizeof(fpgm_ci_result)));
     CK(cudaMemcpyAsync(e->tests_buf.p, tests, (size_t)n_tests * (2 + d) * 4, cudaMemcpyHostToDevice, e->stream));
     CK(cudaMemsetAsync(e->counters.p, 0, kCounterBytes, e->stream));
     CK(cudaMemsetAsync(e->stats.p, 0, ST_COUNT * 8, e->stream));

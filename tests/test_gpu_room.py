@@ -25,7 +25,7 @@ def _check(eng, raw, ref):
     return st
 
 
-@pytest.mark.parametrize("name", ["FPGM_SET_POOL"])
+@pytest.mark.parametrize("name", ["FPGM_SET_POOL", "FPGM_STRATA_POOL"])
 def test_pool_that_cudaMalloc_refuses(monkeypatch, name):
     """cudaMalloc's own refusal (not the engine's cap, which never reaches it) is no error of the
     call: the tests count their own tables."""
@@ -72,6 +72,11 @@ if sys.argv[2] == "sizes":  # device memory of the per-test kernels on these sam
         print(before - torch.cuda.mem_get_info()[0])
     with F.Engine(0) as e:
         print(learn(e, small, sref)["kernel_launches"])
+elif sys.argv[2] == "skeleton":
+    with F.Engine(0) as e:
+        for _ in range(2):
+            learn(e, raw, ref)
+        e.ci_test(0, 1, [2])  # a buffer of 128 MB more
 else:
     with F.Engine(0) as e:
         e.upload(raw)
@@ -81,13 +86,13 @@ else:
 """
 
 
-def _run(what, cap=0):
-    env = dict(os.environ, FPGM_DEVICE_MEM_CAP=str(cap))
+def _run(what, cap=0, **more):
+    env = dict(os.environ, FPGM_DEVICE_MEM_CAP=str(cap), **more)
     return subprocess.run([sys.executable, "-c", _CAPPED, ROOT, what], capture_output=True, text=True, env=env, timeout=600)
 
 
-def _capped(what, cap=0):
-    out = _run(what, cap)
+def _capped(what, cap=0, **more):
+    out = _run(what, cap, **more)
     assert out.returncode == 0, (what, cap, out.stderr[-1500:])
     return [int(v) for v in out.stdout.split()]
 
@@ -97,6 +102,19 @@ def sizes():
     held, launches = _capped("sizes")
     assert held > (1 << 30)
     return held, launches
+
+
+@pytest.mark.parametrize("spare", [20, 60, 100, 160, 240, 500])
+def test_pools_leave_room_for_what_a_skeleton_cannot_do_without(sizes, spare):
+    """Device memory for the per-test kernels and some megabytes more, less than the strata's pool of
+    8,192 sets asks for: a skeleton that succeeds without the pools succeeds with them, and so does a
+    call after it that needs a buffer of its own."""
+    cap = sizes[0] + (spare << 20)
+    alone = _run("skeleton", cap, FPGM_SETS="0", FPGM_STRATA="0", FPGM_BOUND="0")
+    if alone.returncode == 0:
+        _capped("skeleton", cap)
+    else:
+        assert spare < 240 and "FPGM_DEVICE_MEM_CAP" in alone.stderr
 
 
 def test_no_room_for_one_dataset_is_not_kept_for_the_next(sizes):
