@@ -38,6 +38,16 @@ constexpr int kBandDfMax = 1 << 15;   // dense tiers have df < cells <= 24,576
 constexpr uint64_t kEmptyKey = ~0ull;
 
 // ---------------------------------------------------------------- p-value (FP64)
+// ln Gamma without lgamma's write to the process's signgam, on which engines of several threads
+// would race (the host evaluates the p-value of a single test).
+__host__ __device__ inline double ln_gamma(double a) {
+#ifdef __CUDA_ARCH__
+    return lgamma(a);
+#else
+    int sign;
+    return lgamma_r(a, &sign);
+#endif
+}
 // Regularised incomplete gamma from its series (DLMF 8.7.1) and the Legendre continued
 // fraction for Q (DLMF 8.9.2).  One thread evaluates it at the end of a test, so its chain of
 // dependent FP64 operations is what a small test waits for: both are carried as numerator and
@@ -56,7 +66,7 @@ __host__ __device__ inline double igamma_p(double a, double x) {
     const double eps = 1e-16;
     const double big = 0x1p250, small = 0x1p-300;  // eight steps grow the terms by less than 2^300
     const int maxit = 1 << 20;  // times 4 or 8 iterations
-    const double pre = exp(-x + a * log(x) - lgamma(a));
+    const double pre = exp(-x + a * log(x) - ln_gamma(a));
     if (x < (a < 2.0 ? a + 8.0 : a)) {
         // sum of x^n / (a (a + 1) .. (a + n)) = num / den, t = x^n
         double ap = a, den = a, num = 1.0, t = 1.0;
@@ -115,7 +125,7 @@ __host__ __device__ inline double chisq_pvalue(double g2, long long df) {
 __host__ __device__ inline double chisq_pdf(double x, long long df) {
     if (!(x > 0.0)) return df <= 2 ? 1.0 : 0.0;
     const double k = 0.5 * (double)df;
-    return exp((k - 1.0) * log(x) - 0.5 * x - k * 0.69314718055994530942 - lgamma(k));
+    return exp((k - 1.0) * log(x) - 0.5 * x - k * 0.69314718055994530942 - ln_gamma(k));
 }
 
 // Wilson-Hilferty approximation of the upper tail P(chi2_k > x).  Only routes tests

@@ -37,3 +37,15 @@ def test_device_p_value_matches_oracle(card, nz, scale):
     exp = O.ci_tests(cols, cd, tests, nz, threads=1)[0].p_value
     assert r.rechecked == 1
     assert abs(r.p_value - exp) <= 4e-16 * (8 + a * max(1.0, np.log(a + 1)))
+
+
+def test_single_test_leaves_the_process_sign_of_gamma_alone():
+    """The host's part of a single test writes no state of the process (engines run on several
+    threads): the C library's signgam keeps the value it had."""
+    raw, _, _ = F.generate(n_nodes=6, n_samples=2000, seed=4, n_edges=8, max_indegree=3, card=(2, 4))
+    signgam = ctypes.c_int.in_dll(ctypes.CDLL("libm.so.6"), "signgam")
+    with F.Engine(0) as e:
+        e.upload(raw)
+        signgam.value = 77
+        r = e.ci_test(0, 1, [2, 3])
+        assert r.df > 0 and signgam.value == 77
