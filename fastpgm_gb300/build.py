@@ -34,8 +34,8 @@ def nvcc():
 
 
 def _headers():
-    return glob.glob(os.path.join(CSRC, "**", "*.h*"), recursive=True) + glob.glob(
-        os.path.join(ROOT, "include", "*.h"))
+    return [h for pattern in ("*.h", "*.cuh") for h in glob.glob(os.path.join(CSRC, "**", pattern), recursive=True)
+            ] + glob.glob(os.path.join(ROOT, "include", "*.h"))
 
 
 def _stale(obj, src):

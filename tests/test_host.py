@@ -287,3 +287,16 @@ def test_top_level_cmake_example_module():
     out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd="/", env=env)
     assert out.returncode == 0, out.stderr
     assert out.stdout.split() == ["fastpgm_gb300.cmake_example", "True"]
+
+
+def test_every_header_of_the_sources_is_a_dependency_of_the_build():
+    """A unit is rebuilt when a header that it includes is newer, kernels' headers (.cuh) among them."""
+    from fastpgm_gb300 import build
+    known = {os.path.realpath(h) for h in build._headers()}
+    for folder, _, names in os.walk(build.CSRC):
+        for name in names:
+            if name.endswith((".cu", ".cuh", ".cpp", ".h")):
+                for inc in re.findall(r'^#include "([^"]+)"', open(os.path.join(folder, name)).read(), re.M):
+                    found = [p for p in (os.path.join(d, inc) for d in (folder, build.CSRC, os.path.join(ROOT, "include")))
+                             if os.path.exists(p)]
+                    assert found and os.path.realpath(found[0]) in known, (name, inc)
