@@ -11,8 +11,9 @@ CI tests are the reference's deterministic sequential (group size 1) count.
   e2e        same metric through the C ABI with host buffers: upload (H2D + relabel),
              skeleton, result fetch (D2H) inside the timed region
   plain      the same skeleton through the plain one-launch-per-test kernel
-  roofline   counting+scoring kernel: algorithmic bytes (2+|Z|) * n_samples per test over
-             its event-timed duration, against the measured HBM copy bandwidth
+  roofline   counting+scoring kernels: the column bytes their counts read (a set of variables
+             that several tests share once) over their timed duration, against the measured
+             HBM copy bandwidth
   cpu_baseline  the CPU oracle port (reference algorithm, int32 columns, OpenMP) on the host
 
 --impl reference runs the CPU port as the reference arm (rank 0 only).
@@ -320,11 +321,11 @@ def kernel_groups(tot, config, peak, peak_kind):
     the larger share first."""
     kernels = []
     for name, desc, members, ms, nbytes in (
-            ("ci_warp_kernel", "classify + tables shared by variable set (or a test's own), shared memory",
-             ("ci_warp_kernel",), tot["count_ms"], tot["count_bytes"]),
-            ("ci_compact_kernel+ci_part_kernel",
-             "tier 2, joint tables beyond shared memory: hashed strata (compact kernel) and partitioned "
-             "strata (partition kernels)", ("ci_part_kernel", "ci_compact_kernel"), tot["large_ms"],
+            ("set_count_kernel", "classify, then joint tables in shared memory, one per variable set (or a test's "
+             "own), and the tests' scores from them", ("set_count_kernel",), tot["count_ms"], tot["count_bytes"]),
+            ("strata_count_kernel+strata_test_kernel",
+             "joint tables beyond shared memory: shared strata; hashed or partitioned strata (compact and "
+             "partition kernels) of the tests that find no room there", ("strata_count_kernel",), tot["large_ms"],
              tot["large_bytes"])):
         if ms <= 0:
             continue
@@ -332,13 +333,24 @@ def kernel_groups(tot, config, peak, peak_kind):
         tr = profiled_traffic(members, config)
         kernels.append({"kernel": name, "what": desc, "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                         "frac": ach / peak, "peak_kind": peak_kind, "kernel_ms": ms, "algorithmic_bytes": nbytes,
-                        "launches": tot["count_launches"] if name == "ci_warp_kernel" else None,
+                        "launches": tot["count_launches"] if name == "set_count_kernel" else None,
                         "traffic": tr[0] if tr else None,
                         "traffic_source": ("profiles/%s_%s.txt (one ncu capture; not measured in this run)"
                                            % (tr[2], config)) if tr else None,
                         "traffic_launch_algorithmic_bytes": tr[1] if tr else None})
     kernels.sort(key=lambda k: -k["kernel_ms"])
     return kernels
+
+
+def per_test_rate(tot, steps, data):
+    """(2+|Z|) * n_samples for every test run at level >= 1, whether its table was counted for it, shared
+    or not needed, over the counting groups' time: what a count of each test's own would have to
+    read, not a bandwidth.  One dataset only (the statistics do not tell datasets apart)."""
+    ms = tot["count_ms"] + tot["large_ms"]
+    if len(data) != 1 or ms <= 0:
+        return None
+    nbytes = steps * sum(t * (2 + d) * data[0].shape[1] for d, t in enumerate(tot["last"]["tests_executed"]) if d > 0)
+    return {"achieved": nbytes / (ms / 1e3) / 1e9, "unit": "GB/s", "bytes": nbytes}
 
 
 def tensor_peak():
@@ -403,6 +415,7 @@ def north_star_c4(a, l2buf, peak, peak_kind):
            "e2e": {"value": tests / secs, "unit": "CI tests/s", "h2d_bytes_per_step": int(sum(r.nbytes for r in data)),
                    "d2h_bytes_per_step": d2h},
            "counting_phase": counting_phase([(k["kernel_ms"], k["algorithmic_bytes"]) for k in kernels], peak),
+           "per_test_rate": per_test_rate(tot, 2, data),
            "kernel_groups": [{k: g[k] for k in ("kernel", "frac", "kernel_ms", "algorithmic_bytes")} for g in kernels],
            "tensor": gram_roofline(tot),
            "gpu_launches_per_step": tot["kernel_launches"] // 2, "clocks": tot["clocks"]}
@@ -492,6 +505,7 @@ def run_ours(a, d):
     roofline = dict(kernels[0]) if kernels else {"kernel": None}
     roofline["others"] = kernels[1:]
     roofline["counting_phase"] = counting_phase([(k["kernel_ms"], k["algorithmic_bytes"]) for k in kernels], peak)
+    roofline["per_test_rate"] = per_test_rate(tot, a.steps, data)
     roofline["tensor"] = gram_roofline(tot)
     cpu, sample_gpu = None, None
     if d.rank == 0 and d.world == 1 and not a.no_cpu:
@@ -520,7 +534,7 @@ def run_ours(a, d):
         "metric": "CI tests/s (PC-stable skeleton, deterministic test count)", "value": value, "unit": "CI tests/s",
         "n_gpus": a.gpus, "steps": a.steps, "warmup": max(3, a.warmup), "ms_per_step": t_max * 1e3 / a.steps,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "u8 data, int32 counts, fp32 G2 (fp64 p-value and band recheck)",
+        "dtype": "u8 data, int32 counts, 64-bit fixed-point G2 (fp64 terms and p-value where undecided)",
         "data": "synthetic (seeded random DAG + Dirichlet CPTs, forward sampled)",
         "config": bench_config(a, depth),
         "tests_per_step": tot["tests"] // a.steps,

@@ -431,7 +431,8 @@ template <int kSource>
 __global__ void classify_kernel(WaveArgs a) {
     const int T = kSource == SRC_EXPLICIT ? a.n_tests : a.off[a.n_edges];
     const int d = a.d, ncols = d + 2;
-    unsigned long long bytes_shared = 0, bytes_large = 0;  // algorithmic column bytes per tier group
+    // column bytes per tier group: of a test that counts its own table, or of the set it is the first to need
+    unsigned long long bytes_shared = 0, bytes_large = 0;
     for (int item = blockIdx.x * blockDim.x + threadIdx.x; item < T; item += gridDim.x * blockDim.x) {
         int x, y, z[kMaxCond], side = 0;
         if (kSource == SRC_EXPLICIT) {
@@ -499,7 +500,7 @@ __global__ void classify_kernel(WaveArgs a) {
             atomicAdd(&a.stats[ST_UNSUPPORTED], 1ull);
             continue;
         }
-        bool placed = false;
+        bool placed = false, counts = true;  // counts: columns are read for this test here
         if (kSource == SRC_WAVE && tier < 2 && a.sets.key != nullptr) {
             uint16_t sv[kMaxCols];  // the set, ascending (x < y, z ascending)
             for (int k = 0, i = 0, j = 0; k < ncols; ++k) {
@@ -525,6 +526,7 @@ __global__ void classify_kernel(WaveArgs a) {
                         a.sets.fresh[k * a.list_cap + q] = make_int2(at, item);
                     }
                 }
+                counts = fresh && a.sets.off[at] >= 0;
                 const bool warp = work <= a.warp_ints;
                 const int q = atomicAdd(&a.counters[warp ? C_SCOREW : C_SCOREC], 1);
                 a.sets.items[warp ? q : a.list_cap - 1 - q] = make_int2(at, item);
@@ -534,12 +536,13 @@ __global__ void classify_kernel(WaveArgs a) {
         if (placed) {
         } else if (tier == 2 && (side ? dx : dy) <= a.strata_card) {
             a.lists[6 * a.list_cap + atomicAdd(&a.counters[C_STRATA], 1)] = item << 1 | side;
+            counts = false;
         } else {
             const int slot = atomicAdd(&a.counters[C_TIER0 + tier], 1);
             a.lists[tier * a.list_cap + slot] = item;
         }
         const unsigned long long b = (unsigned long long)(2 + d) * (unsigned long long)a.var_S[x];
-        if (tier < 2) bytes_shared += b; else bytes_large += b;
+        if (counts) (tier < 2 ? bytes_shared : bytes_large) += b;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {

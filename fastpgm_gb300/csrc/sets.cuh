@@ -183,6 +183,7 @@ __device__ inline void set_missed(const WaveArgs &a, int item) {
     const int dx = a.card[iv[d]], dy = a.card[iv[d + 1]];
     const int tier = dz * dx * dy + dz * (dx + dy + 1) <= a.warp_ints - 32 ? 0 : 1;
     a.lists[tier * a.list_cap + atomicAdd(&a.counters[C_TIER0 + tier], 1)] = item;
+    atomicAdd(&a.stats[ST_BYTES_SHARED], (unsigned long long)(d + 2) * (unsigned long long)a.var_S[iv[d]]);
 }
 
 // One warp per test, from its set's table.

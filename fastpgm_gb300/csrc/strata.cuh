@@ -244,6 +244,8 @@ __global__ void __launch_bounds__(kStrataThreads, 2) strata_count_kernel(WaveArg
             }
             s_new = 0;
             s_max = 0;
+            if (s_off >= 0)  // ids and column read once, new ids written
+                atomicAdd(&a.stats[ST_BYTES_LARGE], (unsigned long long)S * ((parent < 0 ? 1 : 3) + (kBuild ? 2 : 0)));
         }
         __syncthreads();
         const int64_t off = s_off;
@@ -445,6 +447,7 @@ __global__ void __launch_bounds__(kTestThreads, 5) strata_test_kernel(WaveArgs a
             const int64_t aoff = r0.z >= 0 ? s.pair_a[r0.z] : -1;
             if (n >= 0 && aoff >= 0) {
                 const int nvec = (int)((S + 15) >> 4);
+                if (tid == 0) atomicAdd(&a.stats[ST_BYTES_LARGE], (unsigned long long)S * (2 + m));
                 const uint4 *ids = reinterpret_cast<const uint4 *>(s.pool + s.node_ids[r0.x]);
                 const uint8_t *av = reinterpret_cast<const uint8_t *>(s.pool + aoff);
                 const uint4 *c0 = s_col[0], *c1 = s_col[m > 1 ? 1 : 0], *c2 = s_col[m > 2 ? 2 : 0], *c3 = s_col[m > 3 ? 3 : 0];
@@ -529,6 +532,7 @@ __global__ void __launch_bounds__(kTestThreads, 5) strata_test_kernel(WaveArgs a
                     } else {
                         const int q = atomicAdd(&a.counters[C_TIER2], 1);
                         a.lists[2 * a.list_cap + q] = item;
+                        atomicAdd(&a.stats[ST_BYTES_LARGE], (unsigned long long)S * (2 + d));
                     }
                 }
             }

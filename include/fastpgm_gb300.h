@@ -84,14 +84,15 @@ typedef struct {
     int64_t large_tests;         /* tests counted in global memory */
     double max_abs_dp;           /* max |p32 - p64| over rechecked tests */
     double count_ms;             /* device time of the shared-memory counting+scoring kernel (CUDA events) */
-    double count_bytes;          /* algorithmic bytes its tests read: sum (2+d) * n_samples over the
-                                    tests not decided without a count */
+    double count_bytes;          /* column bytes its counts read: (2+d) * n_samples for each set of variables
+                                    counted, and for each test that counts its own table */
     double large_ms;             /* device time of the global-memory (large table) kernel */
     int64_t count_launches;      /* launches of the counting+scoring kernels */
     int64_t kernel_launches;     /* launches of this library's own kernels (library scans excluded) */
     double span_ms;              /* CUDA-event span of the whole call on the engine's stream */
     double total_ms;             /* host wall time of the whole skeleton call */
-    double large_bytes;          /* algorithmic bytes of the global-memory kernel's tests */
+    double large_bytes;          /* bytes the larger tables' counts read and write: columns and stratum ids of
+                                    each shared set, (2+d) * n_samples for each test that counts alone */
     double gram_ms;              /* device time of level 0 on the tensor cores (one-hot build, Gram GEMM,
                                     pair scoring; 0 when level 0 ran on the counting kernels) */
     double gram_flops;           /* tensor-core flops of that Gram GEMM */
